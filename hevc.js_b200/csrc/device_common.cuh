@@ -30,6 +30,10 @@ static_assert(sizeof(MotionEnt) == 12, "MotionEnt is written as three words by t
 // record and publishes its completion in itu_done.
 constexpr uint32_t INTRA_DEP_EXTERNAL = 0x80000000u;
 constexpr uint32_t INTRA_DEP_WATCH = 0x40000000u;   // | watch slot of the CTU (see ictu_watch)
+constexpr uint32_t INTRA_DEP_INDEX = 0x00FFFFFFu;   // the task index or watch slot
+// Bits 24-28: the parts of the TU's reference array that hold samples of the entry's TU (SEG_*,
+// intra_plan.h); the kernel passes over entries of which the TU's mode reads no part.
+constexpr int INTRA_DEP_SEG_SHIFT = 24;
 constexpr uint8_t ITU_PUBLISH = 1u;
 
 struct PicDesc {
@@ -130,14 +134,5 @@ struct FlowState {
 
 __device__ __forceinline__ int clip3(int lo, int hi, int v) { return v < lo ? lo : (v > hi ? hi : v); }
 __device__ __forceinline__ int clip_u8(int v) { return v < 0 ? 0 : (v > 255 ? 255 : v); }
-
-// 8-bit z-order address of a 4x4 unit inside a CTU (bit-interleave of 4-bit x, y).
-__device__ __forceinline__ uint32_t zorder16(uint32_t bx, uint32_t by) {
-    bx = (bx | (bx << 2)) & 0x33u;
-    bx = (bx | (bx << 1)) & 0x55u;
-    by = (by | (by << 2)) & 0x33u;
-    by = (by | (by << 1)) & 0x55u;
-    return bx | (by << 1);
-}
 
 }  // namespace hevcgpu

@@ -779,10 +779,13 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
         uint32_t* own = owner[c].data();
         const int row = uw[c];
         int dp = 0;
-        uint32_t last = 0;   // a run of units with one owner adds what its first unit added
-        auto dep = [&](uint32_t o) {
-            if ((o & GEN_BITS) != gtag || o == last) return;
+        uint32_t last = 0, last_seg = 0;   // a run of units with one owner adds what its first unit added
+        // seg: the part of b's reference array the unit lies in (SEG_*); an owner's entry carries
+        // all parts it owns samples of
+        auto dep = [&](uint32_t o, uint32_t seg) {
+            if ((o & GEN_BITS) != gtag || (o == last && seg == last_seg)) return;
             last = o;
+            last_seg = seg;
             const int32_t ob = (int32_t)(o & 0xFFFFFFu);
             const int oa = ctu_of[(size_t)ob];
             // a CTU later in raster order is never available to this one
@@ -791,19 +794,24 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
             // yet started: CTAs take CTUs in raster order
             if (oa > a) return;
             for (size_t q = first_dep; q < n_own; q++)
-                if (D[q] == ob) return;
-            D[n_own++] = ob;
+                if ((D[q] & (int32_t)INTRA_DEP_INDEX) == ob) {
+                    D[q] |= (int32_t)(seg << INTRA_DEP_SEG_SHIFT);
+                    return;
+                }
+            D[n_own++] = ob | (int32_t)(seg << INTRA_DEP_SEG_SHIFT);
             dp = std::max(dp, level[(size_t)ob] + 1);   // local and external dependencies alike
         };
         const int ux = t.x / 4, uy = t.y / 4;
         if (t.y > 0) {
             const size_t rrow = (size_t)((t.y - 1) / 4) * row;
             const int ux0 = t.x > 0 ? (t.x - 1) / 4 : 0, ux1 = std::min(row - 1, (t.x + 2 * n - 1) / 4);
-            for (int x = ux0; x <= ux1; x++) dep(own[rrow + x]);
+            const int uxn = ux + n / 4;   // the corner is the unit left of ux
+            for (int x = ux0; x <= ux1; x++) dep(own[rrow + x], x < ux ? SEG_C : (x < uxn ? SEG_T : SEG_TR));
         }
         if (t.x > 0) {
             const int lx = (t.x - 1) / 4, uy0 = t.y / 4, uy1 = std::min(uh[c] - 1, (t.y + 2 * n - 1) / 4);
-            for (int y = uy0; y <= uy1; y++) dep(own[(size_t)y * row + lx]);
+            const int uyn = uy + n / 4;
+            for (int y = uy0; y <= uy1; y++) dep(own[(size_t)y * row + lx], y < uyn ? SEG_L : SEG_BL);
         }
         level[(size_t)b] = dp;
         const uint32_t mark = gtag | (uint32_t)b;
@@ -912,9 +920,10 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
             const int d0 = dep_at[(size_t)b], d1 = dep_at[(size_t)b + 1];
             itu_dep[(size_t)i] = (nd << 6) | (uint32_t)(d1 - d0);
             for (int q = d0; q < d1; q++) {
-                const int ob = deps[(size_t)q], oi = pos[(size_t)ob];
+                const int ob = deps[(size_t)q] & (int32_t)INTRA_DEP_INDEX, oi = pos[(size_t)ob];
+                const uint32_t segs = (uint32_t)deps[(size_t)q] & ~INTRA_DEP_INDEX;
                 if (ctu_of[(size_t)ob] == a) {
-                    dout[nd++] = (uint32_t)(oi - t0);
+                    dout[nd++] = segs | (uint32_t)(oi - t0);
                     continue;
                 }
                 int32_t& so = slot_of[(size_t)oi];
@@ -926,7 +935,7 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
                     watch.push_back((uint32_t)oi);
                     itu_rec[(size_t)oi].reserved[0] = ITU_PUBLISH;
                 }
-                dout[nd++] = INTRA_DEP_WATCH | (uint32_t)(so & 0xFF);
+                dout[nd++] = INTRA_DEP_WATCH | segs | (uint32_t)(so & 0xFF);
             }
             if (!(t.flags & HEVC_TU_CODED)) continue;
             const int nn = 1 << (2 * t.log2_size);
@@ -1220,8 +1229,12 @@ struct Launcher {
 
     template <typename K, typename... A>
     int go(K kernel, dim3 grid, dim3 block, A... args) {
+        return go_smem(kernel, grid, block, 0, args...);
+    }
+    template <typename K, typename... A>
+    int go_smem(K kernel, dim3 grid, dim3 block, size_t smem, A... args) {
         if (grid.x == 0 || grid.y == 0 || grid.z == 0) return HEVCGPU_OK;
-        kernel<<<grid, block, 0, s>>>(args...);
+        kernel<<<grid, block, smem, s>>>(args...);
         ctx->launches++;
         CUDA_TRY(cudaGetLastError());
         return HEVCGPU_OK;
@@ -1366,7 +1379,7 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
             uint32_t* sticky = reinterpret_cast<uint32_t*>(fs + 1);
             int32_t* tickets = ex.tickets();
             CUDA_TRY(cudaMemsetAsync(tickets, 0, sizeof(int32_t) * (size_t)t.n, ex.stream));
-            rc = L.go(k_intra_ctus, dim3(total), dim3(IC_THREADS), t, tickets, total, sticky);
+            rc = L.go_smem(k_intra_ctus, dim3(total), dim3(IC_THREADS), sizeof(IntraSmem), t, tickets, total, sticky);
             if (rc) return rc;
         }
     }
@@ -1466,6 +1479,7 @@ int hevcgpu_create(int device, hevcgpu_ctx_t** out) {
         return fail(HEVCGPU_EUNSUPPORTED, "device %d is sm_%d%d; this library is built for sm_100a", device,
                     prop.major, prop.minor);
     CUDA_TRY(cudaSetDevice(device));
+    CUDA_TRY(cudaFuncSetAttribute(k_intra_ctus, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(IntraSmem)));
     auto* c = new (std::nothrow) hevcgpu_ctx();
     if (!c) return fail(HEVCGPU_ENOMEM, "host allocation");
     c->device = device;
@@ -2007,6 +2021,7 @@ int hevcgpu_intra_schedule(const hevc_picture_syntax_t* syn, hevc_intra_schedule
     if ((rc = build_intra_schedule(BS, syn, &spare))) return rc;
     BS.task_flags.resize(BS.itu_rec.size());
     for (size_t i = 0; i < BS.itu_rec.size(); i++) BS.task_flags[i] = BS.itu_rec[i].reserved[0];
+    for (uint32_t& e : BS.dep_out) e &= INTRA_DEP_WATCH | INTRA_DEP_EXTERNAL | INTRA_DEP_INDEX;   // without the parts
     out->n_ctu = (int32_t)BS.ictu_addr.size();
     out->n_task = (int32_t)BS.intra_list.size();
     out->n_dep = BS.intra_list.empty() ? 0 : (int32_t)spare;   // the entries before the spare one
