@@ -21,20 +21,53 @@ struct MotionEnt {           // 4x4 motion grid entry (PUMotionInfo, inter_predi
 };
 static_assert(sizeof(MotionEnt) == 12, "MotionEnt is written as three words by the MC kernel");
 
-// Intra schedule entries.  Each intra TU in task order has a dependency list: entries
-// without INTRA_DEP_EXTERNAL name a TU of the same CTU by its task index counted from the
-// CTU's first; entries with it name a TU of an earlier CTU of the picture by its task
-// index in the picture (only a planted test wait is left in that form: the host turns
-// each into INTRA_DEP_WATCH | the slot of the CTU's watch list that holds that TU).  A TU
-// that some other CTU depends on carries ITU_PUBLISH in reserved[0] of its task-order
-// record and publishes its completion in itu_done.
+// Intra schedule entries.  Each intra TU in task order has a dependency list: an entry names
+// a TU of the same CTU by its task index counted from the CTU's first, or, with
+// INTRA_DEP_WATCH, a slot of the CTU's watch list, the TUs of earlier CTUs it waits for.
+// (INTRA_DEP_EXTERNAL: a planted test wait.)  A TU that some other CTU depends on carries
+// ITU_PUBLISH in reserved[0] of its task-order record and writes its samples along the CTU's
+// bottom and right into the picture's edge buffer.
 constexpr uint32_t INTRA_DEP_EXTERNAL = 0x80000000u;
-constexpr uint32_t INTRA_DEP_WATCH = 0x40000000u;   // | watch slot of the CTU (see ictu_watch)
-constexpr uint32_t INTRA_DEP_INDEX = 0x00FFFFFFu;   // the task index or watch slot
-// Bits 24-28: the parts of the TU's reference array that hold samples of the entry's TU (SEG_*,
-// intra_plan.h); the kernel passes over entries of which the TU's mode reads no part.
+constexpr uint32_t INTRA_DEP_WATCH = 0x40000000u;   // | watch slot of the CTU: the form handed out
+// The form uploaded: bits 0-8 the source (task index, or IC_MAX_TUS + watch slot), bits 9-17
+// the task that depends on it, bits 24-28 the parts of that task's reference array that hold
+// samples of the source (SEG_*, intra_plan.h): the task does not wait for sources of which
+// its mode reads no part.
+constexpr uint32_t INTRA_DEP_SOURCE = 0x1FFu;
+constexpr int INTRA_DEP_TASK_SHIFT = 9;
 constexpr int INTRA_DEP_SEG_SHIFT = 24;
 constexpr uint8_t ITU_PUBLISH = 1u;
+// A 16x16 or 32x32 TU is done in bands of 8 rows, each by a warp of its own (1,310 and 2,340
+// cycles a band): one warp took 1,770 and 4,200 cycles for the whole TU, a good part of a
+// CTU's chain.
+constexpr int IC_BAND = 8;
+__host__ __device__ constexpr int intra_bands(int log2) { return log2 > 3 ? (1 << log2) / IC_BAND : 1; }
+
+// An intra CTU: its raster address, its TUs in the task order arrays, its entries in the
+// dependency lists and the watch list, its residuals in the residual buffer, its work items,
+// and which neighbour CTUs its TUs may read (NB_*).  Three 16-byte loads.
+struct IntraCtu {
+    int32_t addr, tu_first, n_tu, n_dep;
+    uint32_t dep_first, watch_first;
+    int32_t n_watch;
+    uint32_t nb;
+    int32_t res_first, n_res, item_first, n_item;
+};
+static_assert(sizeof(IntraCtu) == 48, "IntraCtu is read as three 16-byte words");
+
+// Geometry of a watched TU, in units of 4 samples counted from the watching CTU's origin in
+// the TU's plane.
+struct IntraWatch {
+    int c, n4, x4, y4;
+};
+__host__ __device__ __forceinline__ uint32_t intra_watch_pack(const IntraWatch& w) {
+    return (uint32_t)w.c | (uint32_t)w.n4 << 2 | (uint32_t)(w.x4 + 128) << 8 | (uint32_t)(w.y4 + 128) << 16;
+}
+__host__ __device__ __forceinline__ IntraWatch intra_watch_unpack(uint32_t v) {
+    return IntraWatch{(int)(v & 3u), (int)(v >> 2 & 15u), (int)(v >> 8 & 255u) - 128, (int)(v >> 16 & 255u) - 128};
+}
+
+struct IntraTask;   // intra.cuh
 
 struct PicDesc {
     int32_t width, height;               // luma
@@ -47,7 +80,7 @@ struct PicDesc {
     int32_t ref_poc[2][16];
     const hevc_tu_t* tus;
     const int16_t* coeffs;
-    int16_t* resid;                      // residuals of coded intra TUs (at coeff_offset)
+    int16_t* resid;                      // residuals of coded intra TUs, CTU by CTU in task order
     const hevc_pu_t* pus;
     const hevc_wp_t* wp;
     const uint32_t* blk;                 // (W/4)*(H/4)
@@ -57,22 +90,24 @@ struct PicDesc {
     const uint16_t* ctb_tile;            // may be null
     const hevc_slice_t* slices;
     const hevc_scaling_t* scaling;       // scaling lists, or null for flat scaling
-    // intra CTU tasks (intra.cuh): the CTUs that hold intra TUs in wavefront order (key
-    // 2 * row + column), and their TUs ordered by depth in the picture's dependency DAG
-    // (task order)
-    const int32_t* ictu_addr;            // raster address of intra CTU k
-    const int32_t* ictu_tu_off;          // TUs of intra CTU k: task entries [ictu_tu_off[k], [k+1])
+    // intra CTU tasks (intra.cuh): the CTUs that hold intra TUs (IntraCtu, handed to the launch)
+    // in wavefront order (key 2 * row + column), and their TUs ordered by depth in the picture's
+    // dependency DAG (task order)
     const hevc_tu_t* itu_rec;            // TU records in task order; coeff_offset holds the
-                                         // offset of the TU's residual in the CTU's staged ones,
-                                         // reserved[0] ITU_PUBLISH
-    const int4* itu_res;                 // per task entry: residual source offset (-1: none),
-                                         // offset in the CTU's staged residuals, 16-byte chunks
+                                         // offset of the TU's residual in the CTU's, reserved[0]
+                                         // ITU_PUBLISH
+    const int2* itu_res;                 // per task entry of a coded TU: its levels' offset in
+                                         // coeffs, its residual's offset in resid
     const uint32_t* itu_dep;             // per task entry: (offset in dep_list << 6) | count
-    const uint32_t* dep_list;            // dependency entries (INTRA_DEP_EXTERNAL | index)
-    int32_t* itu_done;                   // per task entry: epoch of the launch that completed it
-    const uint32_t* ictu_watch;          // per intra CTU: (offset in watch << 8) | count
-    const uint32_t* watch;               // TUs of other CTUs each CTU waits for (task indices)
-    int32_t n_ictu, n_itu;
+    const uint32_t* dep_list;            // dependency entries
+    const uint16_t* itu_item;            // work items of each CTU: task | band << INTRA_DEP_TASK_SHIFT
+    const uint32_t* watch;               // TUs of other CTUs each CTU waits for (intra_watch_pack)
+    // the plan k_intra_plan makes of them for k_intra_ctus
+    IntraTask* itu_task;
+    uint2* watch_plan;
+    uint16_t* rev;
+    uint8_t* ictu_edge;
+    uint64_t* edge;                      // border words of every CTU, 1 << log2_ctb each
     int32_t num_pus;
     int32_t num_slices;
     int32_t log2_ctb, wctb, hctb;
@@ -87,7 +122,7 @@ struct PicDesc {
 };
 
 // Work items ----------------------------------------------------------------------------
-// Residual items are TU indices (int32); motion-compensation items are packed strips (mc_item, mc.cuh).
+// Residual items are TU indices (int32), or RES_INTRA_ITEM | task index for intra TUs; motion-compensation items are packed strips (mc_item, mc.cuh).
 
 // A launch covers up to MAX_SEGS pictures.  Segment k owns the blocks
 // [block0, next block0) of an item-list launch, or blockIdx.y == k of a per-picture
@@ -113,6 +148,8 @@ __device__ __forceinline__ int find_seg(const SegTable& st, int b) {
     return k;
 }
 
+constexpr uint32_t RES_INTRA_ITEM = 0x80000000u;
+
 // Residual destinations.
 enum ResMode : int32_t {
     RES_PACKED = 0,   // pred/out packed per TU at coeff_offset (config-1 form)
@@ -133,6 +170,14 @@ struct FlowState {
 };
 
 __device__ __forceinline__ int clip3(int lo, int hi, int v) { return v < lo ? lo : (v > hi ? hi : v); }
+// v0..v3 saturated to 0..255 and packed as bytes 0..3 (PTX cvt.pack.sat: the low 16 bits
+// of c move up by 16 and a, b take bits 15..8 and 7..0).
+__device__ __forceinline__ uint32_t pack_sat_u8x4(int v0, int v1, int v2, int v3) {
+    uint32_t t, d;
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, 0;" : "=r"(t) : "r"(v3), "r"(v2));
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(v1), "r"(v0), "r"(t));
+    return d;
+}
 __device__ __forceinline__ int clip_u8(int v) { return v < 0 ? 0 : (v > 255 ? 255 : v); }
 
 }  // namespace hevcgpu

@@ -421,6 +421,10 @@ struct hevcgpu_job {
     int32_t n_mc[2] = {0, 0};            // luma strips, chroma strips (mc.cuh items)
     const uint32_t* d_mc[2] = {nullptr, nullptr};
     int32_t n_ictu = 0;                 // CTUs that hold intra TUs
+    int32_t n_items = 0;                // their work items
+    int32_t depth = 0;                  // TUs of the longest dependency chain
+    const IntraCtu* d_ictu = nullptr;   // their records
+    size_t edge_bytes = 0;              // border words of the intra stage (PicDesc::edge)
     uint32_t spare_dep = 0;             // dependency list entry kept for the planted wait
     int32_t epoch = 0;                  // intra launches of this job so far
     int32_t n_pus = 0;
@@ -594,8 +598,13 @@ struct BuildScratch {
     // clearing only when the 8-bit generation wraps.
     std::vector<uint32_t> owner[3];
     uint32_t gen = 0;
+    int32_t depth = 0;       // TUs of the longest dependency chain
+    int32_t res_total = 0;   // residual samples of the picture's coded intra TUs
     std::vector<hevc_tu_t> itu_rec;
-    std::vector<int4> itu_res;
+    std::vector<int2> itu_res;
+    std::vector<IntraCtu> ictu;
+    std::vector<uint32_t> watch_geo;
+    std::vector<uint16_t> items;
     // intra schedule
     std::vector<int32_t> dep_at, deps, pos, cnt;
     std::vector<std::pair<int64_t, int32_t>> runs;   // (wavefront key, first TU) of each CTU's run
@@ -727,13 +736,17 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
     auto& ictu_watch = BS.ictu_watch;
     ictu_addr.clear();
     ictu_watch.clear();
+    BS.ictu.clear();
     BS.watch.clear();
+    BS.watch_geo.clear();
+    BS.items.clear();
     ictu_tu_off.clear();
     itu.clear();
     itu_rec.clear();
     itu_res.clear();
     itu_dep.clear();
     dep_out.clear();
+    BS.depth = 0;
     if (!n_intra) return HEVCGPU_OK;
     auto& level = BS.level;
     auto& ctu_of = BS.ctu_of;
@@ -759,6 +772,7 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
     }
     const uint32_t gtag = BS.gen << 24;
     constexpr uint32_t GEN_BITS = 0xFF000000u;
+    constexpr int32_t OWNER = 0xFFFFFF;   // of an entry in deps: the owner; above it the parts (SEG_*) it owns
     for (int c = 0; c < 3; c++) {
         uw[c] = (c ? W / 2 : W) / 4;
         uh[c] = (c ? H / 2 : H) / 4;
@@ -794,7 +808,7 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
             // yet started: CTAs take CTUs in raster order
             if (oa > a) return;
             for (size_t q = first_dep; q < n_own; q++)
-                if ((D[q] & (int32_t)INTRA_DEP_INDEX) == ob) {
+                if ((D[q] & OWNER) == ob) {
                     D[q] |= (int32_t)(seg << INTRA_DEP_SEG_SHIFT);
                     return;
                 }
@@ -814,6 +828,7 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
             for (int y = uy0; y <= uy1; y++) dep(own[(size_t)y * row + lx], y < uyn ? SEG_L : SEG_BL);
         }
         level[(size_t)b] = dp;
+        BS.depth = std::max(BS.depth, dp + 1);
         const uint32_t mark = gtag | (uint32_t)b;
         for (int y = uy; y < uy + n / 4; y++) {
             uint32_t* r = own + (size_t)y * row;
@@ -885,19 +900,33 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
     }
     ictu_tu_off.push_back(n_intra);
     // Per CTU in task order: the task-order records (coeff_offset: the TU's offset in the
-    // CTU's staged residuals; reserved[0]: ITU_PUBLISH when a TU of another CTU depends on
-    // it), the residual staging entries and the dependency lists.  A dependency on a TU
+    // CTU's residuals; reserved[0]: ITU_PUBLISH when a TU of another CTU depends on it), where
+    // each coded TU's levels and residual lie, the dependency lists and the CTU's own record.  A dependency on a TU
     // of another CTU goes through the CTU's watcher: the distinct such TUs, in the order
     // their first dependent TU comes, each get a watch slot, and the entry names the slot
     // (INTRA_DEP_WATCH).  Earlier CTUs come first, so the records those entries mark are
     // already written.
-    itu_res.assign((size_t)n_intra, make_int4(-1, 0, 0, 0));
+    itu_res.assign((size_t)n_intra, make_int2(0, 0));
+    int res_total = 0;
     itu_rec.resize((size_t)n_intra);
     itu_dep.resize((size_t)n_intra);
     dep_out.resize(deps.size() + 1);   // one entry per owner found, and the spare entry
     uint32_t* dout = dep_out.data();
     uint32_t nd = 0;
     const int nic = (int)ictu_addr.size();
+    // the neighbour CTBs that share CTB b's slice and tile
+    const uint8_t* slice = s->ctb_slice;
+    const uint16_t* tile = p.tiles_enabled ? s->ctb_tile : nullptr;
+    auto neighbours = [&](int b) -> uint32_t {
+        const int x = b % wctb, y = b / wctb;
+        auto same = [&](int nx, int ny) {
+            if (nx < 0 || ny < 0 || nx >= wctb) return false;
+            const int o = ny * wctb + nx;
+            return (!slice || slice[o] == slice[b]) && (!tile || tile[o] == tile[b]);
+        };
+        return (same(x - 1, y) ? NB_LEFT : 0u) | (same(x - 1, y - 1) ? NB_ABOVE_LEFT : 0u) |
+               (same(x, y - 1) ? NB_ABOVE : 0u) | (same(x + 1, y - 1) ? NB_ABOVE_RIGHT : 0u);
+    };
     auto& watch = BS.watch;
     auto& slot_of = BS.slot_of;   // (CTU index << 8) | slot of a watched TU, by task index
     watch.clear();
@@ -905,7 +934,8 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
     slot_of.assign((size_t)n_intra, -1);
     for (int k = 0; k < nic; k++) {
         int acc = 0, nw = 0;
-        const uint32_t w0 = (uint32_t)watch.size();
+        const uint32_t w0 = (uint32_t)watch.size(), nd0 = nd;
+        const int item0 = (int)BS.items.size();
         const int t0 = ictu_tu_off[(size_t)k], t1 = ictu_tu_off[(size_t)k + 1];
         if (t1 - t0 > IC_MAX_TUS)
             return fail(HEVCGPU_EINVAL, "CTU %d holds more intra TUs than a CTU can", ictu_addr[(size_t)k]);
@@ -920,8 +950,8 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
             const int d0 = dep_at[(size_t)b], d1 = dep_at[(size_t)b + 1];
             itu_dep[(size_t)i] = (nd << 6) | (uint32_t)(d1 - d0);
             for (int q = d0; q < d1; q++) {
-                const int ob = deps[(size_t)q] & (int32_t)INTRA_DEP_INDEX, oi = pos[(size_t)ob];
-                const uint32_t segs = (uint32_t)deps[(size_t)q] & ~INTRA_DEP_INDEX;
+                const int ob = deps[(size_t)q] & OWNER, oi = pos[(size_t)ob];
+                const uint32_t segs = (uint32_t)(deps[(size_t)q] & ~OWNER) | (uint32_t)(i - t0) << INTRA_DEP_TASK_SHIFT;
                 if (ctu_of[(size_t)ob] == a) {
                     dout[nd++] = segs | (uint32_t)(oi - t0);
                     continue;
@@ -933,20 +963,30 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
                                     IC_MAX_WATCH);
                     so = (k << 8) | nw++;
                     watch.push_back((uint32_t)oi);
+                    const hevc_tu_t& o = itu_rec[(size_t)oi];
+                    const int cs = ctb >> (o.c_idx ? 1 : 0);
+                    BS.watch_geo.push_back(intra_watch_pack({o.c_idx, (1 << o.log2_size) / 4, (o.x - a % wctb * cs) / 4,
+                                                             (o.y - a / wctb * cs) / 4}));
                     itu_rec[(size_t)oi].reserved[0] = ITU_PUBLISH;
                 }
-                dout[nd++] = INTRA_DEP_WATCH | segs | (uint32_t)(so & 0xFF);
+                dout[nd++] = segs | (uint32_t)(IC_MAX_TUS + (so & 0xFF));
             }
+            for (int band = 0; band < intra_bands(t.log2_size); band++)
+                BS.items.push_back((uint16_t)((i - t0) | band << INTRA_DEP_TASK_SHIFT));
             if (!(t.flags & HEVC_TU_CODED)) continue;
             const int nn = 1 << (2 * t.log2_size);
-            itu_res[(size_t)i] = make_int4((int)t.coeff_offset, acc, nn / 8, 0);
+            itu_res[(size_t)i] = make_int2((int)t.coeff_offset, res_total + acc);
             r.coeff_offset = (uint32_t)acc;
             acc += nn;
         }
         if (acc > IC_MAX_RES)
             return fail(HEVCGPU_EINVAL, "CTU %d holds more intra TUs than a CTU can", a);
         ictu_watch[(size_t)k] = (w0 << 8) | (uint32_t)nw;
+        BS.ictu.push_back({a, t0, t1 - t0, (int32_t)(nd - nd0), nd0, w0, nw, neighbours(a), res_total, acc, item0,
+                           (int32_t)BS.items.size() - item0});
+        res_total += acc;
     }
+    BS.res_total = res_total;
     // one spare entry: an external dependency of task 0 on itself (the planted wait of
     // hevcgpu_job_plant_unmet_wait points task 0's list at it)
     *spare_dep = nd;
@@ -1043,7 +1083,7 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     for (int i = 0; i < s->num_tus; i++) {
         const hevc_tu_t& t = s->tus[i];
         bool intra = t.flags & HEVC_TU_INTRA;
-        if ((t.flags & HEVC_TU_CODED) && (stages & (intra ? ST_INTRA : ST_RESID))) bins[t.log2_size - 2].push_back(i);
+        if ((t.flags & HEVC_TU_CODED) && !intra && (stages & ST_RESID)) bins[t.log2_size - 2].push_back(i);
         if (intra && (stages & ST_INTRA)) intra_list.push_back(i);
     }
     j->has_intra = !intra_list.empty();
@@ -1057,15 +1097,18 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     // CTUs later in raster order (decoded earlier only in tile scan) are never available
     // and add nothing.
     const int n_intra = (int)intra_list.size();
-    auto& ictu_addr = BS.ictu_addr;
-    auto& ictu_tu_off = BS.ictu_tu_off;
+    auto& ictu = BS.ictu;               // the CTUs' records
     auto& itu_rec = BS.itu_rec;         // intra TU records in task order
-    auto& itu_res = BS.itu_res;         // per task entry: residual source, staged offset, 16-byte chunks
+    auto& itu_res = BS.itu_res;         // per task entry of a coded TU: offsets of its levels and residual
     auto& itu_dep = BS.itu_dep;         // per task entry: (dependency list offset << 6) | count
     auto& dep_out = BS.dep_out;         // dependency lists in task order
-    auto& ictu_watch = BS.ictu_watch;   // per CTU: (offset in watch << 8) | count
     if ((rc = build_intra_schedule(BS, s, &j->spare_dep))) return rc;
-    j->n_ictu = (int32_t)ictu_addr.size();
+    j->n_ictu = (int32_t)ictu.size();
+    j->n_items = (int32_t)BS.items.size();
+    j->depth = BS.depth;
+    for (int i = 0; i < n_intra; i++)
+        if (itu_rec[(size_t)i].flags & HEVC_TU_CODED)
+            bins[itu_rec[(size_t)i].log2_size - 2].push_back((int32_t)(RES_INTRA_ITEM | (uint32_t)i));
     // MC strips (build_mc_strips)
     auto& mc = BS.mc;
     if (stages & ST_MC) build_mc_strips(BS, s, j->lay.pitch_y, j->lay.pitch_c);
@@ -1075,7 +1118,7 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     }
     j->n_pus = s->num_pus;
 
-    size_t o_wp, o_sao, o_sl, o_ti, o_slices, o_res[4], o_mc[2], o_ia, o_idp, o_ito, o_itu, o_iro, o_dl, o_iw, o_wl;
+    size_t o_wp, o_sao, o_sl, o_ti, o_slices, o_res[4], o_mc[2], o_ia, o_idp, o_itu, o_iro, o_dl, o_wl, o_it;
     size_t o_scal = 0;
     hevc_slice_t dflt{0, 0, 0, 1};
     const bool scaled = s->scaling && (stages & (ST_RESID | ST_INTRA));
@@ -1089,14 +1132,13 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
                                                   : pk.add(&dflt, sizeof(dflt));
         for (int k = 0; k < 4; k++) o_res[k] = pk.add(bins[k].data(), sizeof(int32_t) * bins[k].size());
         for (int c = 0; c < 2; c++) o_mc[c] = pk.add(mc[c].data(), sizeof(uint32_t) * mc[c].size());
-        o_ia = pk.add(ictu_addr.data(), sizeof(int32_t) * ictu_addr.size());
-        o_ito = pk.add(ictu_tu_off.data(), sizeof(int32_t) * ictu_tu_off.size());
+        o_ia = pk.add(ictu.data(), sizeof(IntraCtu) * ictu.size());
         o_itu = pk.add(itu_rec.data(), sizeof(hevc_tu_t) * itu_rec.size());
-        o_iro = pk.add(itu_res.data(), sizeof(int4) * itu_res.size());
+        o_iro = pk.add(itu_res.data(), sizeof(int2) * itu_res.size());
         o_idp = pk.add(itu_dep.data(), sizeof(uint32_t) * itu_dep.size());
         o_dl = pk.add(dep_out.data(), sizeof(uint32_t) * dep_out.size());
-        o_iw = pk.add(ictu_watch.data(), sizeof(uint32_t) * ictu_watch.size());
-        o_wl = pk.add(BS.watch.data(), sizeof(uint32_t) * BS.watch.size());
+        o_it = pk.add(BS.items.data(), sizeof(uint16_t) * BS.items.size());
+        o_wl = pk.add(BS.watch_geo.data(), sizeof(uint32_t) * BS.watch_geo.size());
     };
     Packer measure;
     pack(measure);
@@ -1112,10 +1154,20 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     uint8_t* big_base = static_cast<uint8_t*>(j->big.p);
     uint8_t* base = static_cast<uint8_t*>(j->recs.p);
 
-    size_t resid_bytes = j->has_intra ? sizeof(int16_t) * (size_t)align_up((int64_t)s->num_coeffs, 128) : 0;
+    size_t resid_bytes = j->has_intra ? sizeof(int16_t) * (size_t)align_up((int64_t)BS.res_total, 128) : 0;
     size_t mot_bytes = (stages & ST_DEBLOCK) ? sizeof(MotionEnt) * (size_t)align_up((int64_t)gw * gh, 32) : 0;
-    size_t done_bytes = sizeof(int32_t) * (size_t)n_intra;
-    rc = j->scratch.get(ctx, std::max<size_t>(resid_bytes + mot_bytes + done_bytes, 256));
+    // border words of the intra stage, then its plan
+    j->edge_bytes = j->has_intra ? sizeof(uint64_t) * (size_t)nctb * ctb : 0;
+    Packer plan;
+    plan.size = resid_bytes + mot_bytes + j->edge_bytes;
+    size_t o_task = 0, o_wplan = 0, o_rev = 0, o_edge = 0;
+    if (j->has_intra) {
+        o_task = plan.add(nullptr, sizeof(IntraTask) * BS.items.size());
+        o_wplan = plan.add(nullptr, sizeof(uint2) * BS.watch.size());
+        o_rev = plan.add(nullptr, sizeof(uint16_t) * (dep_out.size() + 2));
+        o_edge = plan.add(nullptr, (size_t)IC_EDGES * ictu.size());
+    }
+    rc = j->scratch.get(ctx, std::max<size_t>(plan.size, 256));
     if (rc) return rc;
     rc = j->desc.get(ctx, sizeof(PicDesc));
     if (rc) return rc;
@@ -1144,19 +1196,21 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     D.ctb_tile = (s->ctb_tile && p.tiles_enabled) ? reinterpret_cast<const uint16_t*>(base + o_ti) : nullptr;
     D.slices = reinterpret_cast<const hevc_slice_t*>(base + o_slices);
     D.scaling = scaled ? reinterpret_cast<const hevc_scaling_t*>(base + o_scal) : nullptr;
-    D.ictu_addr = reinterpret_cast<const int32_t*>(base + o_ia);
-    D.ictu_tu_off = reinterpret_cast<const int32_t*>(base + o_ito);
+    j->d_ictu = reinterpret_cast<const IntraCtu*>(base + o_ia);
     D.itu_rec = reinterpret_cast<const hevc_tu_t*>(base + o_itu);
-    D.itu_res = reinterpret_cast<const int4*>(base + o_iro);
+    D.itu_res = reinterpret_cast<const int2*>(base + o_iro);
     D.itu_dep = reinterpret_cast<const uint32_t*>(base + o_idp);
     D.dep_list = reinterpret_cast<const uint32_t*>(base + o_dl);
-    D.ictu_watch = reinterpret_cast<const uint32_t*>(base + o_iw);
+    D.itu_item = reinterpret_cast<const uint16_t*>(base + o_it);
     D.watch = reinterpret_cast<const uint32_t*>(base + o_wl);
-    D.itu_done = reinterpret_cast<int32_t*>(static_cast<uint8_t*>(j->scratch.p) + resid_bytes + mot_bytes);
-    D.n_ictu = (int32_t)ictu_addr.size();
-    D.n_itu = n_intra;
-    // completion flags start below every epoch a launch can use
-    if (done_bytes && (rc = up({UploadOp::ZERO, D.itu_done, nullptr, done_bytes}))) return rc;
+    D.edge = reinterpret_cast<uint64_t*>(static_cast<uint8_t*>(j->scratch.p) + resid_bytes + mot_bytes);
+    uint8_t* const scratch = static_cast<uint8_t*>(j->scratch.p);
+    D.itu_task = reinterpret_cast<IntraTask*>(scratch + o_task);
+    D.watch_plan = reinterpret_cast<uint2*>(scratch + o_wplan);
+    D.rev = reinterpret_cast<uint16_t*>(scratch + o_rev);
+    D.ictu_edge = scratch + o_edge;
+    // border words start below every epoch a launch can use
+    if (j->edge_bytes && (rc = up({UploadOp::ZERO, D.edge, nullptr, j->edge_bytes}))) return rc;
     D.num_pus = s->num_pus;
     D.num_slices = std::max(1, (int)s->num_slices);
     D.log2_ctb = p.log2_ctb;
@@ -1315,6 +1369,17 @@ struct Exec {
     int32_t* tickets() const { return reinterpret_cast<int32_t*>(static_cast<uint8_t*>(flow) + sizeof(FlowState) + 16); }
 };
 
+// Warps per CTU of an intra launch (IC_WIDE or IC_NARROW).  Wide, two CTAs per SM, where the
+// chains of dependent TUs decide: a launch whose deepest picture has `depth` TUs in its
+// longest chain takes about 0.4 us a step.  Narrow, three CTAs per SM, where the number of
+// items does, 1.1 ns each on 148 SMs, and where a CTU has too few for 15 warps.  Measured
+// (us, wide / narrow): 1 and 8 1080p I pictures 482 / 583 and 580 / 687, with 32x32 and 16x16
+// CTBs (4 pictures) 511 / 557 and 854 / 748; 1, 4, 8 and 16 1080p P/B pictures 42 / 49,
+// 59 / 62, 89 / 83 and 142 / 126; 8 with 60 % intra CUs 359 / 415.
+bool intra_wide(int ctus, int64_t items, int depth, int sms) {
+    return items >= 16ll * ctus && (items >= 64ll * ctus || 400ll * depth >= items * 163 / sms);
+}
+
 int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n, int stages, int res_mode) {
     Launcher L{ctx, ex.stream};
     int rc;
@@ -1352,34 +1417,44 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
     if (stages & ST_INTRA) {
         StageMark m(ctx, ex.stream, 3);
         // one launch per group of up to MAX_SEGS pictures: CTAs take intra CTUs by ticket
-        // in (picture, raster) order; aux0 = intra CTUs of earlier pictures, aux1 = epoch
+        // in wavefront order per picture; block0 = intra CTUs of earlier pictures, aux1 = epoch
         int k = 0;
         while (k < n) {
             SegTable t;
             std::memset(&t, 0, sizeof(t));
             int total = 0;
+            int64_t items = 0;
+            int depth = 0;
             for (; k < n && t.n < MAX_SEGS; k++) {
                 hevcgpu_job* j = jobs[k];
                 if (j->n_ictu == 0) continue;
                 Seg& sg = t.s[t.n++];
                 sg.pic = static_cast<const PicDesc*>(j->desc.p);
-                sg.aux0 = total;
-                // completion flags hold the epoch of the launch that set them; restart the
-                // epochs from zero flags before they would reach the sign bit
+                sg.block0 = total;
+                sg.items = j->d_ictu;
+                // border words hold the epoch of the launch that wrote them; restart the epochs
+                // from zero words before they would reach the sign bit
                 if (j->epoch >= 0x7FFFFFF0) {
-                    CUDA_TRY(cudaMemsetAsync(j->host_desc.itu_done, 0, sizeof(int32_t) * (size_t)j->host_desc.n_itu,
-                                             ex.stream));
+                    CUDA_TRY(cudaMemsetAsync(j->host_desc.edge, 0, j->edge_bytes, ex.stream));
                     j->epoch = 0;
                 }
                 sg.aux1 = ++j->epoch;
                 total += j->n_ictu;
+                items += j->n_items;
+                depth = std::max(depth, j->depth);
             }
             if (t.n == 0) continue;
             FlowState* fs = static_cast<FlowState*>(ex.flow);
             uint32_t* sticky = reinterpret_cast<uint32_t*>(fs + 1);
             int32_t* tickets = ex.tickets();
             CUDA_TRY(cudaMemsetAsync(tickets, 0, sizeof(int32_t) * (size_t)t.n, ex.stream));
-            rc = L.go_smem(k_intra_ctus, dim3(total), dim3(IC_THREADS), sizeof(IntraSmem), t, tickets, total, sticky);
+            rc = L.go(k_intra_plan, dim3(total), dim3(IP_THREADS), t, sticky);
+            if (rc) return rc;
+            const bool wide = intra_wide(total, items, depth, ctx->sm_count);
+            rc = wide ? L.go_smem(k_intra_ctus<IC_WIDE>, dim3(total), dim3(32 * IC_WIDE), sizeof(IntraSmem), t, tickets,
+                                  total, sticky)
+                      : L.go_smem(k_intra_ctus<IC_NARROW>, dim3(total), dim3(32 * IC_NARROW), sizeof(IntraSmem), t,
+                                  tickets, total, sticky);
             if (rc) return rc;
         }
     }
@@ -1479,7 +1554,10 @@ int hevcgpu_create(int device, hevcgpu_ctx_t** out) {
         return fail(HEVCGPU_EUNSUPPORTED, "device %d is sm_%d%d; this library is built for sm_100a", device,
                     prop.major, prop.minor);
     CUDA_TRY(cudaSetDevice(device));
-    CUDA_TRY(cudaFuncSetAttribute(k_intra_ctus, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(IntraSmem)));
+    CUDA_TRY(cudaFuncSetAttribute(k_intra_ctus<IC_NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(IntraSmem)));
+    CUDA_TRY(cudaFuncSetAttribute(k_intra_ctus<IC_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(IntraSmem)));
     auto* c = new (std::nothrow) hevcgpu_ctx();
     if (!c) return fail(HEVCGPU_ENOMEM, "host allocation");
     c->device = device;
@@ -2021,7 +2099,10 @@ int hevcgpu_intra_schedule(const hevc_picture_syntax_t* syn, hevc_intra_schedule
     if ((rc = build_intra_schedule(BS, syn, &spare))) return rc;
     BS.task_flags.resize(BS.itu_rec.size());
     for (size_t i = 0; i < BS.itu_rec.size(); i++) BS.task_flags[i] = BS.itu_rec[i].reserved[0];
-    for (uint32_t& e : BS.dep_out) e &= INTRA_DEP_WATCH | INTRA_DEP_EXTERNAL | INTRA_DEP_INDEX;   // without the parts
+    for (uint32_t& e : BS.dep_out) {   // the form the caller reads
+        const uint32_t q = e & INTRA_DEP_SOURCE;
+        e = q < (uint32_t)IC_MAX_TUS ? q : INTRA_DEP_WATCH | (q - (uint32_t)IC_MAX_TUS);
+    }
     out->n_ctu = (int32_t)BS.ictu_addr.size();
     out->n_task = (int32_t)BS.intra_list.size();
     out->n_dep = BS.intra_list.empty() ? 0 : (int32_t)spare;   // the entries before the spare one

@@ -6,21 +6,30 @@
 // residuals ran before).  The host turns that into a dependency list per intra TU: the
 // TUs that own samples of its reference array, in its own CTU (local) or in an earlier CTU
 // (external), and orders each CTU's TUs by their depth in the picture's dependency DAG.
+// k_intra_plan turns that into work items with everything positions and modes tell; then
 // k_intra_ctus runs one CTA per CTU with intra TUs: it stages the CTU with the samples
-// around it, its TU records, dependency lists and residuals in shared memory; its warps take
-// the TUs in order and run each one once the TUs whose samples its mode reads are complete
-// (one-arrival barriers in shared memory for local ones; the CTA's watcher warp follows the
-// flags that other CTUs publish and brings their samples in).  Every wait gives up after
-// WAIT_LIMIT_NS of the GPU's global timer (or SPIN_LIMIT polls, should the timer not
-// advance), sets ST_TIMEOUT in the context's sticky status word (the host turns it into
-// HEVCGPU_ETIMEOUT) and returns.
+// around it, its items and residuals in shared memory; its warps take the items in order and
+// run each one once the TUs whose samples its mode reads are complete (a barrier in shared
+// memory per TU, which counts them; the CTA's watcher warp follows the border words that
+// other CTUs write and brings their samples in).  Every wait gives up after WAIT_LIMIT_NS of
+// the GPU's global timer (or SPIN_LIMIT polls, should the timer not advance), sets ST_TIMEOUT
+// in the context's sticky status word (the host turns it into HEVCGPU_ETIMEOUT) and returns.
 //
-// What bounds it: the chain of dependent TUs, not bytes.  So everything that needs no sample
-// comes before a TU's wait (intra_plan.h: availability, substitution, sample addresses and
-// weights), every sample is read from shared memory after it, and a TU does not wait for
-// samples that its mode does not read (a 1080p I picture's longest chain: 860 TUs instead of
-// 2167).  Batch of 8 1080p I pictures: 1.18 ms, 2.18 ms with the waits on every owner and the
-// work after the wait.
+// What bounds it: the chain of dependent TUs and, in P/B pictures, the instructions per TU;
+// not bytes.  So
+//   - a TU waits only for TUs whose samples its mode reads (a 1080p I picture's longest chain
+//     is 860 TUs; 2167 with every owner of its reference array);
+//   - everything that needs no sample comes before its wait (intra_plan.h: availability,
+//     substitution, sample addresses and weights), every sample is read from shared memory;
+//   - a completed TU arrives at the TUs that wait for it, so a wait is one barrier (185 cycles
+//     when it is met already, 97 from the last arrival; 550 and 270 when each TU tested the
+//     barriers of all it depends on);
+//   - samples cross CTU borders with their flag in one 64-bit word, with no fence on either
+//     side;
+//   - the code is small: what does not run per TU is a kernel of its own, since instruction
+//     cache misses were half of all stalls with it inside.
+// 8 1080p I pictures: 0.58 ms, 2.18 with waits on every owner and the work after the wait; 1 and
+// 16 1080p P/B pictures 43 and 126 us, 107 and 276 then.
 #pragma once
 
 #include <cuda/atomic>
@@ -30,39 +39,19 @@
 
 namespace hevcgpu {
 
-__constant__ int8_t c_intra_angle[35] = {0,   0,   32,  26,  21,  17,  13,  9,  5,  2,  0,  -2,
-                                         -5,  -9,  -13, -17, -21, -26, -32, -26, -21, -17, -13, -9,
-                                         -5,  -2,  0,   2,   5,   9,   13,  17,  21,  26,  32};
-__constant__ int16_t c_inv_angle[35] = {0,    0,    256, 315, 390, 482,  630,  910,  1638, 4096, 0,   4096,
-                                        1638, 910,  630, 482, 390, 315,  256,  315,  390,  482,  630, 910,
-                                        1638, 4096, 0,   4096, 1638, 910, 630, 482,  390,  315,  256};
+__device__ const IntraTapTable c_intra_taps = intra_tap_table();
+__constant__ IntraAngles c_intra = intra_angles();
 
-
-// The picture fields a TU reads, copied into shared memory once per CTA: reads of the
-// descriptor in global memory would go through L1, which every GPU-scope acquire on the SM
-// invalidates, and sit in each TU's chain of dependent loads.
-struct IntraPic {
-    uint8_t* rec;
-    int64_t off_cb, off_cr;
-    int32_t width, height, log2_ctb, pitch_y, pitch_c, intra_smoothing_disabled, strong_intra;
-};
-
-// A warp's reference samples of an 8x8..32x32 TU, in main order (mirrored for the
-// horizontal modes, so that the main side always runs upwards from index 2n): as read, and
-// smoothed and / or projected.
+// A warp's reference samples of an 8x8..32x32 TU, in main order: mirrored for the horizontal
+// modes, so that the main side always runs upwards from index 2n.
 struct alignas(4) IntraWarpSmem {
-    uint8_t raw[132];   // 4n + 1 samples
-    uint8_t ref[132];   // the smoothed array, or main entries q = -n .. 2n + 1 at [q + n]
+    uint8_t ref[136];   // 4n + 1 samples, and what aligned reads of them reach past the end
 };
 
-// One plane of the CTU in shared memory with the samples around it that its TUs read: the
-// column left of it, the corner, and the row above as far as the end of the above-right
-// CTU.  Sample (x, y) counted from the CTU's origin is at t[y * pitch + x]; only row -1
-// reaches past the CTU's width.
-struct CtuTile {
-    uint8_t* t;
-    int pitch, x0, y0;
-};
+// A plane of the CTU lies in shared memory as a tile with the samples around it that its TUs
+// read: the column left of it, the corner, and the row above as far as the end of the
+// above-right CTU.  Sample (x, y) counted from the CTU's origin is at origin[y * pitch + x];
+// only row -1 reaches past the CTU's width.
 
 // Address (offset from the CTU's origin in its tile) of reference sample k of a TU whose
 // origin is at offset o.
@@ -76,146 +65,137 @@ __device__ __forceinline__ uint32_t dp4a_uu(uint32_t a, uint32_t b, uint32_t c) 
     return d;
 }
 
-// The 4x4 TU (most TUs, and most of a picture's dependency chain): one output sample per lane
-// (x = lane & 3, y = lane >> 2; the upper half of the warp repeats the lower), each from four
-// samples of the tile whose addresses and weights are known before the wait (IntraTaps4), so
-// that what follows it is four shared loads, a weighted sum and a store.  4x4 references are
-// never smoothed (:217-230 and :443-445).  done() completes the TU: the tile holds its
-// samples; the store to the picture follows it, off the chain.
-// In a 1080p I picture a TU takes 150 cycles after its wait; 980 when samples were fetched by
-// lane and moved by shuffles, other CTUs' samples read through L2, and the substitution found
-// with ballots.
-template <typename Wait, typename Done>
-__device__ __forceinline__ bool intra_tu4(const IntraPic& P, const hevc_tu_t& t, uint32_t av_word, int lane,
-                                          const CtuTile& tile, const int16_t* res, Wait&& wait, Done&& done) {
-    const bool chroma = t.c_idx != 0;
-    const int x = lane & 3, y = (lane >> 2) & 3, mode = t.intra_mode;
-    const IntraAvail av = avail_unpack(av_word, 4);
-    const IntraTaps4 k = intra_taps4(mode, chroma, x, y, lane, c_intra_angle[mode], c_inv_angle[mode]);
-    const int o = (t.y - tile.y0) * tile.pitch + (t.x - tile.x0);
-    const bool none = avail_segs(av) == 0u;   // no reference sample: every one is 128
-    int at[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) at[j] = none ? 0 : ref_offset(o, tile.pitch, 4, intra_substitute(av, k.i[j]));
-    const int r = res != nullptr ? res[lane & 15] : 0;
-    const bool pcm = (t.flags & HEVC_TU_PCM) != 0;
-    uint8_t* const plane = P.rec + (t.c_idx == 0 ? 0 : (t.c_idx == 1 ? P.off_cb : P.off_cr));
-    const int pitch = chroma ? P.pitch_c : P.pitch_y;
-    if (!wait()) return false;
-    int v[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) v[j] = none ? 128 : (int)tile.t[at[j]];
-    if (mode == 1) v[1] = (int)(__reduce_add_sync(0xffffffffu, lane < 8 ? v[1] : 0) + 4) >> 3;
-    int p = clip_u8((v[0] * k.w[0] + v[1] * k.w[1] + v[2] * k.w[2] + v[3] * k.w[3] + k.add) >> k.shift);
-    if (pcm) p = 0;   // the PCM samples are the levels, with no prediction
-    const uint8_t out = (uint8_t)clip_u8(p + r);
-    if (lane < 16) tile.t[o + y * tile.pitch + x] = out;
-    done();
-    if (lane < 16) plane[(int64_t)(t.y + y) * pitch + t.x + x] = out;
-    return true;
+// A work item as k_intra_plan lays it down for the warp that runs it (32 bytes), a TU or one
+// band of it: where its samples lie, what stands in for reference samples that are not
+// available, what it waits for and who waits for it.
+struct alignas(16) IntraTask {
+    uint32_t pic;          // offset of the TU's first sample in the picture buffer
+    uint32_t source;       // (first << 16) | count of the TUs that wait for the TU, in rev
+    uint16_t tile;         // offset of its first sample in the CTU's tiles
+    uint16_t res;          // offset of its residual in the CTU's residuals (zeros for a 4x4 TU without one)
+    int16_t first, corner; // the first available reference sample and the one that stands at
+                           // the corner, as tile offsets from its first sample
+    uint8_t mode, flags;   // 0..34 or MODE_PCM; TASK_*
+    uint8_t log2, y0;      // the TU's size; first row of the band
+    int8_t angle;
+    uint8_t waits;         // arrivals the TU's barrier takes
+    uint8_t bl, tr;        // available samples below-left and top-right
+    uint8_t row, column;   // its first border word along the CTU's bottom / right, or TASK_NO_EDGE
+    int16_t inv_angle;
+    uint16_t bar, pad;     // its barrier: the task index
+};
+static_assert(sizeof(IntraTask) == 32, "IntraTask is copied as two 16-byte words");
+constexpr uint8_t TASK_NO_EDGE = 0xFF;
+enum : uint8_t {
+    TASK_CHROMA = 1, TASK_CODED = 2, TASK_SMOOTH = 4, TASK_LEFT = 8, TASK_TOP = 16,   // left / top available
+    TASK_STARTED = 32,   // waits for nothing: its barrier starts complete
+};
+
+// Tile offset, from the TU's first sample, of the sample that stands at index i of its
+// reference array (intra_substitute; the constant 128 when none is available).
+__device__ __forceinline__ int task_where(const IntraTask& t, int n, int pitch, int i) {
+    const bool top = t.flags & TASK_TOP;
+    const int left = t.flags & TASK_LEFT ? (2 * n - 1 - plan_max(i, n - t.bl)) * pitch - 1 : t.first;
+    const int along = plan_min(i, 3 * n + t.tr) - 2 * n - 1 - pitch;
+    return i < 2 * n ? left : (i > (top ? 2 * n : 3 * n) && (top || t.tr) ? along : t.corner);
 }
 
-// The 8x8, 16x16 and 32x32 TU (perform_intra_prediction, then reconstruct_block's add and
-// clip), one copy of the code for the three sizes to keep the kernel small in the instruction
-// cache.  After the wait the substituted reference array goes from the tile to the warp's
-// shared memory in main order; smoothing and the projection of the side reference, where the
-// mode has them, make one more pass over it; then each lane predicts groups of 4 samples of a
-// row (its column is the same for all its groups).  done() as in intra_tu4, after the stores.
-template <typename Wait, typename Done>
-__device__ __forceinline__ bool intra_tu(const IntraPic& P, const hevc_tu_t& t, uint32_t av_word, int lane,
-                                         IntraWarpSmem& W, const CtuTile& tile, const int16_t* res, Wait&& wait,
-                                         Done&& done) {
-    constexpr int RMAX = 5;   // lane rounds of the largest reference array
-    const int log2 = t.log2_size, n = 1 << log2, total = 4 * n + 1, mode = t.intra_mode;
-    const bool chroma = t.c_idx != 0, vert = mode >= 18 || mode < 2;
-    const IntraAvail av = avail_unpack(av_word, n);
-    const bool none = avail_segs(av) == 0u;
-    const bool smooth = intra_smoothed(mode, log2, chroma, P.intra_smoothing_disabled != 0);
-    const int ang = c_intra_angle[mode], inv = c_inv_angle[mode];
-    const int o = (t.y - tile.y0) * tile.pitch + (t.x - tile.x0);
-    int at[RMAX];   // where sample i = lane + 32 r of the array in main order lies
-#pragma unroll
-    for (int r = 0; r < RMAX; r++) {
-        const int i = plan_min(lane + 32 * r, 4 * n);
-        at[r] = none ? 0 : ref_offset(o, tile.pitch, n, intra_substitute(av, vert ? i : 4 * n - i));
-    }
-    const int gpr = n >> 2, x0 = 4 * (lane & (gpr - 1)), ystep = 32 >> (log2 - 2);
-    int cidx[4], cw[4];   // horizontal modes: the columns' offsets and weights
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        cidx[j] = ((x0 + j + 1) * ang) >> 5;
-        cw[j] = ((x0 + j + 1) * ang) & 31;
-    }
-    const bool edge = !chroma && n < 32, pcm = (t.flags & HEVC_TU_PCM) != 0;
-    uint8_t* const plane = P.rec + (t.c_idx == 0 ? 0 : (t.c_idx == 1 ? P.off_cb : P.off_cr));
-    const int pitch = chroma ? P.pitch_c : P.pitch_y;
-    if (!wait()) return false;
-
+// Rows y0 .. y0 + rows - 1 of an 8x8 (smoothed), 16x16 or 32x32 TU (perform_intra_prediction,
+// then reconstruct_block's add and clip) into the tile, one copy of the code for the three
+// sizes.  The substituted reference array comes from the tile into registers, sample
+// lane + 32 r in lane `lane` and the last one in every lane, is smoothed there and goes to the
+// warp's shared memory in main order; for a negative angle the side reference is projected in
+// front of the main one, in place; then each lane predicts groups of 4 samples of a row.
+// at[r]: where sample lane + 32 r lies (r < 2); at_end: where sample 4n lies.
+__device__ __forceinline__ void intra_predict(const IntraTask& task, int strong_intra, int lane, uint8_t* ref,
+                                              int at0, int at1, int at_end, uint8_t* t, int pitch, int y0, int rows,
+                                              const int16_t* res, bool coded) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    const int log2 = task.log2, n = 1 << log2, mode = task.mode, ang = task.angle;
+    const bool vert = mode >= 18 || mode < 2, smooth = task.flags & TASK_SMOOTH;
+    const bool edge = !(task.flags & TASK_CHROMA) && log2 < 5;
     // 1. the substituted reference array (:177-197)
+    int v[4], end = t[at_end];
+    v[0] = t[at0];
+    v[1] = v[2] = v[3] = 0;
+    if (log2 > 3) v[1] = t[at1];
+    if (log2 > 4) {
 #pragma unroll
-    for (int r = 0; r < RMAX; r++) {
-        const int i = lane + 32 * r;
-        if (i < total) W.raw[i] = none ? (uint8_t)128 : tile.t[at[r]];
+        for (int r = 2; r < 4; r++)
+            v[r] = t[task_where(task, n, pitch, vert ? lane + 32 * r : 4 * n - lane - 32 * r)];
     }
-    __syncwarp();
     // 2. smoothing of luma references (:217-257, :443-471): [1 2 1] over the array, ends
-    //    kept, or the bilinear strong smoothing of 32x32; and for the modes with a negative
-    //    angle the main reference with the side reference projected (:346-368)
-    int ro = 0, mo = 2 * n;   // offsets from W.raw: the array in main order, main reference entry 0
-    if (smooth || ang < 0) {
-        const int c = W.raw[2 * n], e0 = W.raw[0], e1 = W.raw[4 * n];
-        const bool strong = smooth && n == 32 && P.strong_intra && abs(c + e1 - 2 * W.raw[3 * n]) < 8 &&
-                            abs(c + e0 - 2 * W.raw[n]) < 8;
-        const int count = ang < 0 ? 3 * n + 2 : total;
-        for (int e = lane; e < count; e += 32) {
-            const int i = ang < 0 ? intra_main_index(true, inv, n, e - n) : e;
-            int f = W.raw[i];
-            if (smooth && i != 0 && i != 4 * n) {
-                if (strong) {
-                    const int d = i > 2 * n ? i - 2 * n : 2 * n - i;   // from the corner (0: the corner itself)
-                    f = ((2 * n - d) * c + d * (i > 2 * n ? e1 : e0) + n) >> (log2 + 1);
-                } else {
-                    f = (W.raw[i - 1] + 2 * f + W.raw[i + 1] + 2) >> 2;
+    //    kept, or the bilinear strong smoothing of 32x32
+    if (smooth) {
+        const int rounds = 1 << (log2 - 3);
+        int f[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            f[r] = v[r];
+            if (r >= rounds) continue;
+            const int down = __shfl_sync(FULL, v[r], (lane + 31) & 31), up = __shfl_sync(FULL, v[r], (lane + 1) & 31);
+            const int below = r > 0 ? __shfl_sync(FULL, v[r > 0 ? r - 1 : 0], 31) : v[0];
+            const int above = r + 1 < rounds ? __shfl_sync(FULL, v[r < 3 ? r + 1 : 3], 0) : end;
+            if (r > 0 || lane > 0) f[r] = ((lane ? down : below) + 2 * v[r] + (lane < 31 ? up : above) + 2) >> 2;
+        }
+        if (log2 == 5 && strong_intra) {
+            const int e0 = __shfl_sync(FULL, v[0], 0), c = __shfl_sync(FULL, v[2], 0);
+            if (abs(c + end - 2 * __shfl_sync(FULL, v[3], 0)) < 8 && abs(c + e0 - 2 * __shfl_sync(FULL, v[1], 0)) < 8) {
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const int i = lane + 32 * r, d = abs(i - 64);   // from the corner
+                    if (i > 0) f[r] = ((64 - d) * c + d * (i > 64 ? end : e0) + 32) >> 6;
                 }
             }
-            W.ref[e] = (uint8_t)f;
         }
-        __syncwarp();
-        ro = (int)sizeof(W.raw);
-        mo = ro + (ang < 0 ? n : 2 * n);   // with a negative angle only the main entries are read
+#pragma unroll
+        for (int r = 0; r < 4; r++) v[r] = f[r];
     }
-    const uint8_t* const R = W.raw + ro;
-    const uint8_t* const M = W.raw + mo;
-    // 3. prediction + residual, clip, store
+    ref[lane] = (uint8_t)v[0];
+    if (log2 > 3) ref[lane + 32] = (uint8_t)v[1];
+    if (log2 > 4) {
+        ref[lane + 64] = (uint8_t)v[2];
+        ref[lane + 96] = (uint8_t)v[3];
+    }
+    if (lane == 0) ref[4 * n] = (uint8_t)end;
+    __syncwarp();
+    // 3. for a negative angle, main entries -1 .. -n: the side reference projected through
+    //    invAngle (:346-368)
+    if (ang < 0) {
+        const int side = ref[2 * n - plan_min(2 * n, ((lane + 1) * task.inv_angle + 128) >> 8)];
+        __syncwarp();
+        if (lane < n) ref[2 * n - 1 - lane] = (uint8_t)side;
+        __syncwarp();
+    }
+    // 4. prediction + residual, clip, store
     int dc = 0;
     if (mode == 1) {   // predict_dc :295-317
-        int sum = 0;
-        if (lane < n) sum = R[2 * n + 1 + lane] + R[2 * n - 1 - lane];
-        sum = __reduce_add_sync(0xffffffffu, sum);
-        dc = (sum + n) >> (log2 + 1);
+        dc = (int)__reduce_add_sync(FULL, lane < n ? ref[2 * n + 1 + lane] + ref[2 * n - 1 - lane] : 0);
+        dc = (dc + n) >> (log2 + 1);
     }
-    const int corner = M[0];
-    for (int y = lane >> (log2 - 2); y < n; y += ystep) {
+    const int x0 = 4 * (lane & ((n >> 2) - 1));
+#pragma unroll 1
+    for (int y = y0 + (lane >> (log2 - 2)); y < y0 + rows; y += 128 >> log2) {
+        int2 rw = make_int2(0, 0);   // residual: four int16 in one 8-byte load
+        if (coded) rw = *reinterpret_cast<const int2*>(res + y * n + x0);
         int p[4];
-        if (mode == 0) {   // predict_planar :263-289
-            const int left = R[2 * n - 1 - y], tr = R[3 * n + 1], bl = R[n - 1];
+        if (mode < 2) {   // planar (:263-289) or DC with its edge rows
+            const int left = ref[2 * n - 1 - y], tr = ref[3 * n + 1], bl = ref[n - 1];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const int x = x0 + j;
-                p[j] = ((n - 1 - x) * left + (x + 1) * tr + (n - 1 - y) * R[2 * n + 1 + x] + (y + 1) * bl + n) >>
-                       (log2 + 1);
+                const int x = x0 + j, top = ref[2 * n + 1 + x];
+                p[j] = mode == 0 ? ((n - 1 - x) * left + (x + 1) * tr + (n - 1 - y) * top + (y + 1) * bl + n) >> (log2 + 1)
+                       : edge && y == 0 ? (top + 3 * dc + 2) >> 2
+                                        : dc;
             }
-        } else if (mode == 1) {
-            const int left = R[2 * n - 1 - y];
-#pragma unroll
-            for (int j = 0; j < 4; j++) p[j] = edge && y == 0 ? (R[2 * n + 1 + x0 + j] + 3 * dc + 2) >> 2 : dc;
-            if (edge && x0 == 0) p[0] = y == 0 ? (R[2 * n + 1] + left + 2 * dc + 2) >> 2 : (left + 3 * dc + 2) >> 2;
+            if (mode == 1 && edge && x0 == 0)
+                p[0] = y == 0 ? (ref[2 * n + 1] + left + 2 * dc + 2) >> 2 : (left + 3 * dc + 2) >> 2;
         } else if (vert) {   // predict_angular :323-422, main reference on top
             // entries q .. q + 4 of the main reference as bytes of two realigned words; sample j
             // weighs bytes j and j + 1
             const int idx = ((y + 1) * ang) >> 5, fr = ((y + 1) * ang) & 31;
-            const int a = mo + x0 + 1 + idx;
-            const uint32_t* const words = reinterpret_cast<const uint32_t*>(W.raw) + (a >> 2);
+            const int a = 2 * n + x0 + 1 + idx;
+            const uint32_t* const words = reinterpret_cast<const uint32_t*>(ref) + (a >> 2);
             const uint32_t w0 = words[0], w1 = words[1];
             const uint32_t lo = __funnelshift_r(w0, w1, 8 * (a & 3)), hi = w1 >> (8 * (a & 3));
             const uint32_t wt = (uint32_t)(32 - fr) | ((uint32_t)fr << 8);
@@ -223,57 +203,37 @@ __device__ __forceinline__ bool intra_tu(const IntraPic& P, const hevc_tu_t& t, 
             p[1] = (int)(dp4a_uu(lo, wt << 8, 16u) >> 5);
             p[2] = (int)(dp4a_uu(lo, wt << 16, 16u) >> 5);
             p[3] = (int)(dp4a_uu(__funnelshift_r(lo, hi, 24), wt, 16u) >> 5);
-            if (edge && mode == 26 && x0 == 0) p[0] = clip_u8(p[0] + ((R[2 * n - 1 - y] - corner) >> 1));
+            if (edge && mode == 26 && x0 == 0) p[0] = clip_u8(p[0] + ((ref[2 * n - 1 - y] - ref[2 * n]) >> 1));
         } else {   // main reference on the left
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const uint8_t* m = M + y + 1 + cidx[j];
-                p[j] = ((32 - cw[j]) * m[0] + cw[j] * m[1] + 16) >> 5;
-            }
-            if (edge && mode == 10 && y == 0) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) p[j] = clip_u8(p[j] + ((R[2 * n - 1 - x0 - j] - corner) >> 1));
+                const int idx = ((x0 + j + 1) * ang) >> 5, fr = ((x0 + j + 1) * ang) & 31;
+                const uint8_t* m = ref + 2 * n + y + 1 + idx;
+                p[j] = ((32 - fr) * m[0] + fr * m[1] + 16) >> 5;
+                if (edge && mode == 10 && y == 0) p[j] = clip_u8(p[j] + ((ref[2 * n - 1 - x0 - j] - ref[2 * n]) >> 1));
             }
         }
-        if (pcm) {   // the PCM samples are the levels, with no prediction
-#pragma unroll
-            for (int j = 0; j < 4; j++) p[j] = 0;
-        }
-        // residual (four int16 in one 8-byte load), clip, one word to the tile and the picture
-        if (res != nullptr) {
-            const int2 rw = *reinterpret_cast<const int2*>(res + y * n + x0);
-            p[0] = clip_u8(p[0] + (int)(int16_t)(rw.x & 0xFFFF));
-            p[1] = clip_u8(p[1] + (rw.x >> 16));
-            p[2] = clip_u8(p[2] + (int)(int16_t)(rw.y & 0xFFFF));
-            p[3] = clip_u8(p[3] + (rw.y >> 16));
-        }
-        const uint32_t w = (uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24);
-        *reinterpret_cast<uint32_t*>(tile.t + o + y * tile.pitch + x0) = w;
-        *reinterpret_cast<uint32_t*>(plane + (int64_t)(t.y + y) * pitch + t.x + x0) = w;
+        if (mode == MODE_PCM) p[0] = p[1] = p[2] = p[3] = 0;
+        *reinterpret_cast<uint32_t*>(t + y * pitch + x0) =
+            pack_sat_u8x4(p[0] + (int)(int16_t)(rw.x & 0xFFFF), p[1] + (rw.x >> 16), p[2] + (int)(int16_t)(rw.y & 0xFFFF),
+                          p[3] + (rw.y >> 16));
     }
-    done();
-    return true;
 }
 
 // ---------------------------------------------------------------------------------------
 // CTU tasks.  One CTA per CTU that holds intra TUs.  CTAs take CTUs by ticket in wavefront
 // order per picture (2 * row + column: the diagonal band along which a picture's
-// dependencies advance), the pictures of a launch side by side.  The CTA stages the CTU with
-// the samples around it, its TU records and their residuals in shared memory; then its warps
-// take the TUs one at a time in task order (by depth in the picture's DAG, so every TU comes
-// after the TUs it depends on) and run each as soon as the TUs whose samples it reads are
-// complete: a TU of the same CTU through its one-arrival barrier in shared memory, a TU of
-// an earlier CTU through that TU's published completion in global memory.  No barrier ties
-// the warps together, so the critical path is the chain of dependent TUs itself.  Every wait
-// is for a TU taken earlier, by this CTA or by a CTA holding an earlier ticket, which is
-// already running; every wait is bounded.  The CTA's last warp is its watcher: it alone
-// polls the global flags of the TUs of other CTUs and copies their samples into the tile's
-// border, so the workers only read shared memory and wait on shared-memory barriers, which
-// suspend them without taking issue slots.
+// dependencies advance), the pictures of a launch side by side.  The CTA's warps take the
+// items one at a time in task order (by depth in the picture's DAG, so every TU comes after
+// the TUs it depends on).  No barrier ties the warps together, so the critical path is the
+// chain of dependent TUs itself.  Every wait is for a TU taken earlier, by this CTA or by a
+// CTA holding an earlier ticket, which is already running.  The CTA's last warp is its
+// watcher: it alone polls words of other CTUs, so the workers only read shared memory and
+// wait on shared-memory barriers, which suspend them without taking issue slots.
 // ---------------------------------------------------------------------------------------
-constexpr int IC_WARPS = 8;
-constexpr int IC_THREADS = 32 * IC_WARPS;
-constexpr int IC_MIN_BLOCKS = 3;
+// Warps of a CTA (the last one watches): IC_WIDE where the chains decide, IC_NARROW where the
+// number of CTUs does (intra_wide).
+constexpr int IC_NARROW = 8, IC_WIDE = 16;
 // Tiles: a margin of 16 bytes (its last byte is the column left of the CTU; 16 keeps the
 // CTU's rows on 16-byte boundaries for the asynchronous copies), the CTU, the CTU to the
 // right (row -1 only); row -1 first.  Pitches that are odd multiples of 16 spread a column
@@ -285,7 +245,12 @@ constexpr int IC_MAX_TUS = 256 + 2 * 64;             // 4x4 TUs of a 64x64 CTU, 
 constexpr int IC_MAX_RES = 64 * 64 + 2 * 32 * 32;    // residual samples of a 64x64 CTU
 constexpr int IC_DEP_STAGE = 2048;                   // dependency entries staged per CTU
 constexpr int IC_MAX_WATCH = 128;                    // TUs of other CTUs a CTU waits for
-constexpr int IC_WORKERS = IC_WARPS - 1;             // worker warps; the last warp watches
+constexpr int IC_SOURCES = IC_MAX_TUS + IC_MAX_WATCH;   // what a TU can wait for: TUs here, watched TUs
+// Border words (4 samples) a CTU's TUs can read, per plane: the corner, the row above over two
+// CTUs, the column to the left.
+constexpr int IC_EDGE_L = 1 + 3 * 16, IC_EDGE_C = 1 + 3 * 8;
+constexpr int IC_EDGES = 128;                        // >= IC_EDGE_L + 2 * IC_EDGE_C, 4 per watcher lane
+constexpr int IC_TILES = IC_LH * IC_LP + 2 * IC_CH * IC_CP;   // bytes of the three tiles; then a byte 128
 constexpr unsigned long long WAIT_LIMIT_NS = 1000000000ull;   // a wait gives up after a second
 constexpr unsigned SPIN_LIMIT = 1u << 26;            // backstop: polls of at least 64 ns
 
@@ -301,32 +266,26 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
                  "l"(gmem));
 }
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem));
+}
 __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
-// One-arrival barriers in shared memory, one per TU of the CTU: the warp that completes
-// the TU arrives (release), the warps whose TUs read its samples wait on phase 0 (acquire).
-// A waiting thread is suspended by the hardware until the phase completes or the time hint
-// runs out, so waiting warps take no issue slots from the working ones.
-__device__ __forceinline__ void mbar_init1(uint64_t* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(bar)) : "memory");
+// Barriers in shared memory, one per TU of the CTU that waits for others, with as many
+// arrivals as the TUs it waits for: each arrives when it completes (release), the TU's warp
+// waits on phase 0 (acquire).  A waiting thread is suspended by the hardware until the phase
+// completes or the time hint runs out, so waiting warps take no issue slots from the working
+// ones.
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t arrivals) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(arrivals)
+                 : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.release.cta.shared::cta.b64 st, [%0];\n\t}" ::"r"(
                      (uint32_t)__cvta_generic_to_shared(bar))
                  : "memory");
-}
-// whether phase 0 of the barrier has completed, without waiting
-__device__ __forceinline__ bool mbar_test0(uint64_t* bar) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cta.shared::cta.b64 p, [%1], 0;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"((uint32_t)__cvta_generic_to_shared(bar))
-        : "memory");
-    return ok != 0;
 }
 // true once phase 0 of the barrier has completed; false when the time hint ran out first
 __device__ __forceinline__ bool mbar_try_wait0(uint64_t* bar) {
@@ -340,53 +299,40 @@ __device__ __forceinline__ bool mbar_try_wait0(uint64_t* bar) {
     return ok != 0;
 }
 
-// Copy plane c of CTU (rx, ry) and the samples around it into its tile (16-byte copies are
-// issued, not waited for).  Samples of other CTUs that an intra TU still has to write come
-// again with that TU's completion (the watcher); all others are final.
-__device__ __forceinline__ void stage_tile(const PicDesc& P, int c, int rx, int ry, uint8_t* origin, int tid,
-                                           int threads) {
-    const int sub = c ? 2 : 1, ctbc = (1 << P.log2_ctb) / sub;
-    const int pw = P.width / sub, ph = P.height / sub, pitch = c ? P.pitch_c : P.pitch_y;
-    const uint8_t* plane = P.rec + (c == 0 ? 0 : (c == 1 ? P.off_cb : P.off_cr));
+// Copy plane c of CTU (rx, ry) and the samples around it into its tile (copies issued, not
+// waited for).  Samples of other CTUs that an intra TU still has to write come again as
+// border words (the watcher); all others are final.
+template <int THREADS>
+__device__ __forceinline__ void stage_tile(const PicDesc& P, int c, int rx, int ry, uint8_t* origin, int tid) {
+    const int sub = c ? 1 : 0, log2c = P.log2_ctb - sub, cs = 1 << log2c;
+    const int pw = P.width >> sub, ph = P.height >> sub, pitch = c ? P.pitch_c : P.pitch_y;
+    const uint8_t* const plane = P.rec + (c == 0 ? 0 : (c == 1 ? P.off_cb : P.off_cr));
     const int tp = c ? IC_CP : IC_LP;
-    const int x0 = rx * ctbc, y0 = ry * ctbc;
-    if (ctbc >= 16) {
-        // rows 0 .. ctbc - 1, then the row above over two CTUs (a 16-byte piece that starts
+    const int x0 = rx << log2c, y0 = ry << log2c;
+    if (log2c >= 4) {
+        // rows 0 .. cs - 1, then the row above over two CTUs (a 16-byte piece that starts
         // inside the picture ends inside the row's pitch, a multiple of 64)
-        const int row_chunks = ctbc / 16, own = ctbc * row_chunks;
-        for (int e = tid; e < own + 2 * row_chunks; e += threads) {
-            const int r = e < own ? e / row_chunks : -1, q = e < own ? e % row_chunks : e - own;
+        const int per_row = log2c - 4, own = cs << per_row;
+#pragma unroll 1
+        for (int e = tid; e < own + (2 << per_row); e += THREADS) {
+            const int r = e < own ? e >> per_row : -1, q = e < own ? e & ((1 << per_row) - 1) : e - own;
             const int y = y0 + r, x = x0 + 16 * q;
-            if (y < 0 || y >= ph || x >= pw) continue;
-            cp_async16(origin + r * tp + 16 * q, plane + (int64_t)y * pitch + x);
+            if (y >= 0 && y < ph && x < pw) cp_async16(origin + r * tp + 16 * q, plane + (int64_t)y * pitch + x);
         }
     } else {  // 8-sample chroma CTBs (16x16 CTUs): words
-        for (int e = tid; e < ctbc * 2 + 4; e += threads) {
-            const int r = e < ctbc * 2 ? e / 2 : -1, q = e < ctbc * 2 ? e % 2 : e - ctbc * 2;
+#pragma unroll 1
+        for (int e = tid; e < 8 * 2 + 4; e += THREADS) {
+            const int r = e < 16 ? e >> 1 : -1, q = e < 16 ? e & 1 : e - 16;
             const int y = y0 + r, x = x0 + 4 * q;
-            if (y < 0 || y >= ph || x >= pw) continue;
-            *reinterpret_cast<uint32_t*>(origin + r * tp + 4 * q) =
-                __ldcg(reinterpret_cast<const uint32_t*>(plane + (int64_t)y * pitch + x));
+            if (y >= 0 && y < ph && x < pw) cp_async4(origin + r * tp + 4 * q, plane + (int64_t)y * pitch + x);
         }
     }
-    if (rx > 0)   // the corner and the column to the left
-        for (int r = tid - 1; r < ctbc; r += threads) {
-            const int y = y0 + r;
-            if (y >= 0 && y < ph) origin[r * tp - 1] = __ldcg(plane + (int64_t)y * pitch + x0 - 1);
-        }
+    // the corner and the column to the left, as the words that end there
+    if (rx > 0 && tid <= cs) {
+        const int y = y0 + tid - 1;
+        if (y >= 0 && y < ph) cp_async4(origin + (tid - 1) * tp - 4, plane + (int64_t)y * pitch + x0 - 4);
+    }
 }
-
-// The state one worker's wait for a TU's dependencies reads.
-struct IntraWait {
-    const uint32_t* s_dep;      // the CTU's staged dependency entries
-    const uint32_t* dep_list;   // all entries (those past the staged ones)
-    uint64_t* s_bar;            // completion barriers of the CTU's TUs, then its watch barriers
-    int32_t* itu_done;          // published completions (direct external entries)
-    uint32_t* sticky;
-    volatile int* s_abort;
-    int dfirst, doff, dcount, staged, task, n_watch, n_itu, epoch, lane;
-    uint32_t need;              // the parts of the reference array the TU reads (SEG_*)
-};
 
 // True while the wait that began at t0 may go on (t0 = 0: it begins now).
 __device__ __forceinline__ bool wait_goes_on(unsigned long long& t0, unsigned polls, uint32_t* sticky,
@@ -399,92 +345,209 @@ __device__ __forceinline__ bool wait_goes_on(unsigned long long& t0, unsigned po
     return false;
 }
 
-// A direct external entry: polls the published completion (only a planted test wait has one).
-__device__ __noinline__ bool wait_published(int32_t* flag, int epoch, uint32_t* sticky, volatile int* s_abort) {
-    cuda::atomic_ref<int32_t, cuda::thread_scope_device> f(*flag);
-    unsigned long long t0 = 0;
-    for (unsigned polls = 0; f.load(cuda::memory_order_relaxed) != epoch; polls++) {
-        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> status(*sticky);
-        if (!wait_goes_on(t0, polls, sticky, s_abort) || (status.load(cuda::memory_order_relaxed) & ST_TIMEOUT))
-            return false;
-        __nanosleep(64);
-    }
-    cuda::atomic_thread_fence(cuda::memory_order_acquire, cuda::thread_scope_device);
-    return true;
+// Lane 0's claim of the next work item, one instruction with no branch around it; the other
+// lanes get 0.
+__device__ __forceinline__ uint32_t claim_item(int* next, int lane) {
+    uint32_t v;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %2, 0;\n\tmov.u32 %0, 0;\n\t@p atom.shared.add.u32 %0, [%1], 1;\n\t}"
+        : "=&r"(v)
+        : "r"((uint32_t)__cvta_generic_to_shared(next)), "r"(lane)
+        : "memory");
+    return v;
 }
 
-// The wait for a TU's dependencies, between the position work and the loads of a TU path:
-// each lane tests one entry's barrier, entries whose TU wrote nothing the mode reads are
-// passed over, and while some are pending the warp is suspended as a whole on the pending one
-// with the greatest index (watched TUs come after local ones, local ones by depth), which
-// is mostly the last to complete.  Testing the entries one after the other cost 130 cycles
-// each.  Every wait reads the global timer and gives up after WAIT_LIMIT_NS (SPIN_LIMIT tries
-// as a backstop), marking the sticky status; a wait also ends when another warp of the CTA
-// gave up (s_abort) or, for external waits, when a wait anywhere did (the status word).
-__device__ __forceinline__ bool intra_wait(const IntraWait& w) {
-    constexpr uint32_t FULL = 0xffffffffu;
-    bool gave_up = false;
-    for (int base = 0; base < w.dcount && !gave_up; base += 32) {
-        const int q = base + w.lane, at = w.doff + q;
-        uint32_t bar = 0;   // 1 + index of the barrier this lane's entry waits for, 0 when it does not
-        if (q < w.dcount) {
-            const uint32_t e = at >= 0 && at < w.staged ? w.s_dep[at] : __ldg(&w.dep_list[w.dfirst + at]);
-            const uint32_t k = e & INTRA_DEP_INDEX;
-            if (e & INTRA_DEP_EXTERNAL) {
-                if (k < (uint32_t)w.n_itu) {
-                    gave_up = !wait_published(&w.itu_done[k], w.epoch, w.sticky, w.s_abort);
-                } else {
-                    atomicOr(w.sticky, ST_BAD_RECORD);
-                    gave_up = true;
+// Border words of one CTU in the picture's edge buffer, ctb of them per CTU in raster order:
+// the bottom row's words (Y, Cb, Cr), then the right column's.  A word holds 4 samples and
+// the epoch of the launch that wrote them, stored and read whole: a reader that finds its
+// epoch has the samples too, with no fence on either side and no second read.
+__device__ __forceinline__ int edge_word(int ctb, int c, bool column, int i) {
+    return (column ? ctb >> 1 : 0) + (c == 0 ? 0 : (c == 1 ? ctb >> 2 : (ctb >> 2) + (ctb >> 3))) + i;
+}
+
+// Offset of the CTU's origin in each plane's tile (IntraSmem: luma, Cb, Cr tiles one after
+// the other).
+__device__ __forceinline__ int tile_origin(int c) {
+    return c == 0 ? IC_LP + IC_MARGIN : IC_LH * IC_LP + (c - 1) * (IC_CH * IC_CP) + IC_CP + IC_MARGIN;
+}
+
+// ---------------------------------------------------------------------------------------
+// The plan of a CTU's tasks, one CTA per CTU: which samples each TU can and does read, for
+// how many TUs it waits, and for each TU and watched TU ("source") the TUs that wait for it.
+// It follows from the records alone, so it is a launch of its own before the samples are
+// needed: inside k_intra_ctus it took 5,500 to 16,000 of a CTU's cycles and its code pushed
+// the TU paths out of the instruction caches (no_instruction 5.5 of 11 stall cycles per
+// instruction; 0.7 of 6 now).
+//   itu_task[item]    the work items
+//   watch_plan[...]   per watched TU: its waiting TUs as in IntraTask::source, and its border words
+//   rev[...]          task indices counted from the CTU's first, at dep_first
+//   ictu_edge[...]    per border word the watch slot whose sample it awaits, or 0xFF
+// ---------------------------------------------------------------------------------------
+constexpr int AV_WAITS_SHIFT = 16;           // s_av: avail_pack; bits 16-21 the arrivals the TU waits for
+constexpr uint32_t AV_UNMET = 1u << 22;      // a planted test wait: an arrival that never comes
+constexpr int AV_NEED_SHIFT = 23;            // bits 23-27 the parts of its reference array it reads
+constexpr int AV_BANDS_SHIFT = 28;           // bits 28-30 its bands
+constexpr int IP_THREADS = 128;
+
+__global__ void __launch_bounds__(IP_THREADS) k_intra_plan(const __grid_constant__ SegTable st, uint32_t* sticky) {
+    __shared__ uint32_t s_av[IC_MAX_TUS], s_count[IC_SOURCES], s_fill[IC_SOURCES], s_total, s_bad;
+    __shared__ uint8_t s_edge[IC_EDGES];
+    const int tid = threadIdx.x, lane = tid % 32;
+    const int k = find_seg(st, blockIdx.x);
+    const PicDesc& P = *st.s[k].pic;
+    const int idx = blockIdx.x - st.s[k].block0;
+    const IntraCtu C = static_cast<const IntraCtu*>(st.s[k].items)[idx];
+    const int n_tu = min(C.n_tu, IC_MAX_TUS), n_watch = min(C.n_watch, IC_MAX_WATCH);
+#pragma unroll 1
+    for (int q = tid; q < IC_SOURCES; q += IP_THREADS) s_count[q] = 0;
+    if (tid < IC_EDGES) s_edge[tid] = 0xFF;
+    if (tid == 0) s_total = s_bad = 0;
+#pragma unroll 1
+    for (int i = tid; i < n_tu; i += IP_THREADS) {
+        const hevc_tu_t t = P.itu_rec[C.tu_first + i];
+        const uint32_t dd = P.itu_dep[C.tu_first + i], at = dd >> 6;
+        const int c = t.c_idx != 0;
+        const IntraAvail av =
+            intra_avail(t.x, t.y, 1 << t.log2_size, P.width >> c, P.height >> c, P.log2_ctb - c, 1 + c, C.nb);
+        const bool smooth = intra_smoothed(t.intra_mode, t.log2_size, c, P.intra_smoothing_disabled != 0);
+        const uint32_t need =
+            intra_need(intra_parts(t.intra_mode, t.log2_size, c, (t.flags & HEVC_TU_PCM) != 0, smooth), avail_segs(av));
+        // a list outside the CTU's entries is a planted one
+        const bool planted = (dd & 63u) && (at < C.dep_first || at >= C.dep_first + (uint32_t)C.n_dep) &&
+                             (P.dep_list[at] & INTRA_DEP_EXTERNAL);
+        s_av[i] = avail_pack(av) | (planted ? AV_UNMET : 0u) | (need << AV_NEED_SHIFT) |
+                  ((uint32_t)intra_bands(t.log2_size) << AV_BANDS_SHIFT);
+    }
+    __syncthreads();
+    // the entries whose TU wrote something the waiting TU's mode reads.  Refused: an entry that
+    // names no earlier TU and no watch slot, or no task of the CTU
+    auto read = [&](int q, int& i, int& s) {
+        const uint32_t e = __ldg(&P.dep_list[C.dep_first + q]);
+        s = (int)(e & INTRA_DEP_SOURCE);
+        i = (int)((e >> INTRA_DEP_TASK_SHIFT) & INTRA_DEP_SOURCE);
+        if (i >= n_tu || s >= (s < IC_MAX_TUS ? i : IC_MAX_TUS + n_watch)) {
+            s_bad = 1;
+            return false;
+        }
+        return ((e >> INTRA_DEP_SEG_SHIFT) & (s_av[i] >> AV_NEED_SHIFT) & SEG_ALL) != 0;
+    };
+#pragma unroll 1
+    for (int q = tid; q < C.n_dep; q += IP_THREADS) {
+        int i, s;
+        if (read(q, i, s)) {
+            atomicAdd(&s_count[s], 1u);
+            atomicAdd(&s_av[i], (s < IC_MAX_TUS ? s_av[s] >> AV_BANDS_SHIFT : 1u) << AV_WAITS_SHIFT);   // one per band
+        }
+    }
+    __syncthreads();
+    // room in rev for each source's waiting TUs (sources in any order: a warp takes its
+    // sources' room at once), and the border words the watched TUs stand for
+#pragma unroll 1
+    for (int s = tid; s < IC_SOURCES; s += IP_THREADS) {
+        const uint32_t count = s_count[s];
+        uint32_t end = count;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, end, d);
+            if (lane >= d) end += v;
+        }
+        uint32_t first = 0;
+        if (lane == 31 && end) first = atomicAdd(&s_total, end);
+        first = __shfl_sync(0xffffffffu, first, 31) + end - count;
+        s_fill[s] = first;
+        s_count[s] = (first << 16) | count;
+        const int j = s - IC_MAX_TUS;
+        if (j >= 0 && j < n_watch) {
+            const IntraWatch w = intra_watch_unpack(P.watch[C.watch_first + j]);
+            const int cw = (1 << (P.log2_ctb - (w.c ? 1 : 0))) / 4;   // words across the CTU
+            uint8_t* const edge = s_edge + (w.c == 0 ? 0 : IC_EDGE_L + (w.c - 1) * IC_EDGE_C);
+            const int left0 = 1 + 2 * (w.c ? 8 : 16);
+            uint32_t n = 0;
+#pragma unroll 1
+            for (int u = 0; u < w.n4 && count; u++) {
+                if (w.y4 + w.n4 == 0 && w.x4 + u >= -1 && w.x4 + u < 2 * cw) {
+                    edge[1 + w.x4 + u] = (uint8_t)j;
+                    n++;
                 }
-            } else if ((e >> INTRA_DEP_SEG_SHIFT) & w.need) {
-                if (k < (uint32_t)((e & INTRA_DEP_WATCH) ? w.n_watch : w.task)) {
-                    bar = 1 + ((e & INTRA_DEP_WATCH) ? IC_MAX_TUS + k : k);
-                    if (mbar_test0(&w.s_bar[bar - 1])) bar = 0;
-                } else {
-                    atomicOr(w.sticky, ST_BAD_RECORD);   // not an earlier TU, or no such watch slot: refused
-                    gave_up = true;
+                if (w.x4 + w.n4 == 0 && w.y4 + u >= 0 && w.y4 + u < cw) {
+                    edge[left0 + w.y4 + u] = (uint8_t)j;
+                    n++;
                 }
             }
-        }
-        gave_up = __any_sync(FULL, gave_up);
-        unsigned long long t0 = 0;
-        uint32_t last = __reduce_max_sync(FULL, bar);
-        for (unsigned polls = 0; last != 0u && !gave_up; polls++) {
-            if (!mbar_try_wait0(&w.s_bar[last - 1])) gave_up = !wait_goes_on(t0, polls, w.sticky, w.s_abort);
-            if (bar != 0u && mbar_test0(&w.s_bar[bar - 1])) bar = 0;
-            last = __reduce_max_sync(FULL, bar);
-            // the lanes may have seen the barrier, the abort word or the clock at different moments
-            gave_up = __any_sync(FULL, gave_up);
+            P.watch_plan[C.watch_first + j] = make_uint2((first << 16) | count, n);
+            if (count && n == 0) s_bad = 1;   // not beside this CTU: refused
         }
     }
-    // the warp barrier orders each lane's acquires before every lane's reads of the samples
-    __syncwarp();
-    return !gave_up;
+    __syncthreads();
+#pragma unroll 1
+    for (int q = tid; q < C.n_dep; q += IP_THREADS) {
+        int i, s;
+        if (read(q, i, s)) P.rev[C.dep_first + atomicAdd(&s_fill[s], 1u)] = (uint16_t)i;
+    }
+#pragma unroll 1
+    for (int q = tid; q < C.n_item; q += IP_THREADS) {
+        const int item = P.itu_item[C.item_first + q], i = item & (int)INTRA_DEP_SOURCE, band = item >> INTRA_DEP_TASK_SHIFT;
+        const hevc_tu_t t = P.itu_rec[C.tu_first + i];
+        const int c = t.c_idx, sub = c ? 1 : 0, n = 1 << t.log2_size, cs = 1 << (P.log2_ctb - sub);
+        const int x = t.x & (cs - 1), y = t.y & (cs - 1), tp = c ? IC_CP : IC_LP, pitch = c ? P.pitch_c : P.pitch_y;
+        const IntraAvail a = avail_unpack(s_av[i], n);
+        const bool coded = t.flags & HEVC_TU_CODED, publish = t.reserved[0] & ITU_PUBLISH, pcm = t.flags & HEVC_TU_PCM;
+        const bool none = avail_segs(a) == 0u;
+        const int waits = (int)(s_av[i] >> AV_WAITS_SHIFT & 63u) + (s_av[i] & AV_UNMET ? 1 : 0), ctb = 1 << P.log2_ctb;
+        IntraTask k;
+        k.pic = (uint32_t)((c == 0 ? 0 : (c == 1 ? P.off_cb : P.off_cr)) + (int64_t)t.y * pitch + t.x);
+        k.source = s_count[i];
+        k.tile = (uint16_t)(tile_origin(c) + y * tp + x);
+        k.res = coded ? (uint16_t)t.coeff_offset : (uint16_t)IC_MAX_RES;
+        k.first = (int16_t)(none ? IC_TILES - k.tile : ref_offset(0, tp, n, intra_substitute(a, 0)));
+        k.corner = (int16_t)(none ? IC_TILES - k.tile : ref_offset(0, tp, n, intra_substitute(a, 2 * n)));
+        k.mode = pcm ? (uint8_t)MODE_PCM : t.intra_mode;
+        const bool smooth = !pcm && intra_smoothed(t.intra_mode, t.log2_size, c != 0, P.intra_smoothing_disabled != 0);
+        k.flags = (uint8_t)((c ? TASK_CHROMA : 0) | (coded ? TASK_CODED : 0) | (smooth ? TASK_SMOOTH : 0) |
+                            (a.l ? TASK_LEFT : 0) | (a.t ? TASK_TOP : 0) | (waits ? 0 : TASK_STARTED));
+        k.log2 = t.log2_size;
+        k.y0 = (uint8_t)(band * IC_BAND);
+        k.angle = pcm ? 0 : c_intra.angle[t.intra_mode];
+        k.inv_angle = pcm ? 0 : c_intra.inv[t.intra_mode];
+        k.waits = (uint8_t)plan_max(waits, 1);
+        k.bl = (uint8_t)a.bl;
+        k.tr = (uint8_t)a.tr;
+        k.row = publish && y + n == cs ? (uint8_t)edge_word(ctb, c, false, x / 4) : TASK_NO_EDGE;
+        k.column = publish && x + n == cs ? (uint8_t)edge_word(ctb, c, true, y / 4) : TASK_NO_EDGE;
+        k.bar = (uint16_t)i;
+        k.pad = 0;
+        P.itu_task[C.item_first + q] = k;
+    }
+    if (tid < IC_EDGES / 4)
+        reinterpret_cast<uint32_t*>(P.ictu_edge)[idx * (IC_EDGES / 4) + tid] = reinterpret_cast<const uint32_t*>(s_edge)[tid];
+    if (tid == 0 && s_bad) atomicOr(sticky, ST_BAD_RECORD);   // k_intra_ctus then does nothing
 }
 
+// ---------------------------------------------------------------------------------------
+// The CTU tasks themselves.
+// ---------------------------------------------------------------------------------------
 // A CTA's shared memory (dynamic: more than 48 KB).
 struct IntraSmem {
-    alignas(16) uint8_t t_luma[IC_LH * IC_LP];
-    alignas(16) uint8_t t_chroma[2][IC_CH * IC_CP];
-    alignas(16) hevc_tu_t tu[IC_MAX_TUS];
-    alignas(16) int16_t res[IC_MAX_RES];
-    alignas(16) hevc_tu_t wtu[IC_MAX_WATCH];   // records of the watched TUs of other CTUs
-    uint64_t bar[IC_MAX_TUS + IC_MAX_WATCH];   // completion of the CTU's TUs, by task index, then of the watched ones
-    IntraWarpSmem ws[IC_WORKERS];
-    uint32_t av[IC_MAX_TUS];        // available and needed reference samples (avail_pack)
-    uint32_t itu_dep[IC_MAX_TUS];   // dependency lists: (offset << 6) | count
-    uint32_t dep[IC_DEP_STAGE];     // the CTU's dependency entries
-    uint32_t watch[IC_MAX_WATCH];   // the watched TUs' task indices in the picture
-    uint32_t wneed[IC_MAX_WATCH / 32];   // those whose samples some TU reads
-    IntraPic pic;
-    uint32_t nb;
+    alignas(16) uint8_t tiles[IC_TILES + 16];   // and the constant 128, for TUs with no reference sample
+    alignas(16) IntraTask task[IC_MAX_TUS];     // the CTU's part of PicDesc::itu_task
+    alignas(16) int16_t res[IC_MAX_RES + 16];   // and the residual of 4x4 TUs without one
+    alignas(16) uint2 taps[36 * 2 * 16];        // c_intra_taps
+    alignas(16) uint8_t edge[IC_EDGES];     // PicDesc::ictu_edge
+    alignas(16) uint16_t rev[IC_DEP_STAGE + 2];   // the CTU's part of PicDesc::rev
+    uint64_t bar[IC_MAX_TUS];               // what each TU waits for
+    uint2 watch[IC_MAX_WATCH];              // PicDesc::watch_plan, y counted down as border words come
+    IntraWarpSmem ws[IC_WIDE - 1];
     int ticket, pic_index, next;
     volatile int abort;
 };
+static_assert(IC_LH * IC_LP % 16 == 0 && IC_CH * IC_CP % 16 == 0, "the tiles' rows lie on 16-byte boundaries");
 
-__global__ void __launch_bounds__(IC_THREADS, IC_MIN_BLOCKS) k_intra_ctus(const __grid_constant__ SegTable st,
-                                                                       int32_t* tickets, int total, uint32_t* sticky) {
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 24 / WARPS + (WARPS > 8)) k_intra_ctus(const __grid_constant__ SegTable st,
+                                                                                 int32_t* tickets, int total,
+                                                                                 uint32_t* sticky) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    constexpr int THREADS = 32 * WARPS;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     IntraSmem& S = *reinterpret_cast<IntraSmem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
@@ -495,225 +558,288 @@ __global__ void __launch_bounds__(IC_THREADS, IC_MIN_BLOCKS) k_intra_ctus(const 
         // CTA finds one.
         int k = blockIdx.x % st.n, got = -1;
         for (int tries = 0; tries < st.n && got < 0; tries++) {
-            const int n_k = (k + 1 < st.n ? st.s[k + 1].aux0 : total) - st.s[k].aux0;
+            const int n_k = (k + 1 < st.n ? st.s[k + 1].block0 : total) - st.s[k].block0;
             const int v = atomicAdd(&tickets[k], 1);
             if (v < n_k) got = v;
             else k = k + 1 == st.n ? 0 : k + 1;
         }
-        // a wait of this launch (or an earlier one not yet read) gave up: the CTU could only
-        // wait for work that will not come, so the CTA ends at once
-        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> status(*sticky);
-        S.ticket = (status.load(cuda::memory_order_relaxed) & ST_TIMEOUT) ? -1 : got;
+        S.ticket = got;
         S.pic_index = k;
-        S.abort = 0;
         S.next = 0;
     }
-    if (tid < IC_MAX_WATCH / 32) S.wneed[tid] = 0;
+    if (tid == 32) {
+        // a wait of this launch (or an earlier one not yet read) gave up, or the plan was
+        // refused: the CTU could only wait for work that will not come, so the CTA ends at once
+        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> status(*sticky);
+        S.abort = status.load(cuda::memory_order_relaxed) != 0;
+    }
+#pragma unroll 1
+    for (int q = tid; q < (int)sizeof(S.taps) / 16; q += THREADS)
+        cp_async16(reinterpret_cast<uint4*>(S.taps) + q, reinterpret_cast<const uint4*>(c_intra_taps.t) + q);
     __syncthreads();
-    if (S.ticket < 0) return;
+    if (S.ticket < 0 || S.abort) {
+        cp_async_wait_all();
+        return;
+    }
     const int k = S.pic_index;
     const PicDesc& P = *st.s[k].pic;
     const int32_t epoch = st.s[k].aux1;
-    const int idx = S.ticket;
-    const int a = P.ictu_addr[idx], rx = a % P.wctb, ry = a / P.wctb;
+    // the CTU's record: the same 16-byte loads by every thread, and no chain of loads after it
+    const int4* const cp = reinterpret_cast<const int4*>(static_cast<const IntraCtu*>(st.s[k].items) + S.ticket);
+    const int4 c0 = __ldg(cp), c1 = __ldg(cp + 1), c2 = __ldg(cp + 2);
+    const int a = c0.x, n_dep = min(c0.w, IC_DEP_STAGE), n_watch = min(c1.z, IC_MAX_WATCH);
+    const int n_res = min(c2.y, IC_MAX_RES), n_item = min(c2.w, IC_MAX_TUS);
+    const int rx = a % P.wctb, ry = a / P.wctb, ctbl = 1 << P.log2_ctb;
 
-    if (tid == 32) {
-        S.pic.rec = P.rec;
-        S.pic.off_cb = P.off_cb;
-        S.pic.off_cr = P.off_cr;
-        S.pic.width = P.width;
-        S.pic.height = P.height;
-        S.pic.log2_ctb = P.log2_ctb;
-        S.pic.pitch_y = P.pitch_y;
-        S.pic.pitch_c = P.pitch_c;
-        S.pic.intra_smoothing_disabled = P.intra_smoothing_disabled;
-        S.pic.strong_intra = P.strong_intra;
-    }
-    if (tid == 4) {  // which neighbour CTBs share this CTB's slice and tile
-        const int sl = P.ctb_slice ? P.ctb_slice[a] : 0, ti = P.ctb_tile ? P.ctb_tile[a] : 0;
-        auto same = [&](int nx, int ny) {
-            if (nx < 0 || ny < 0 || nx >= P.wctb) return false;
-            const int b = ny * P.wctb + nx;
-            return (P.ctb_slice ? P.ctb_slice[b] : 0) == sl && (P.ctb_tile ? P.ctb_tile[b] : 0) == ti;
-        };
-        S.nb = (same(rx - 1, ry) ? NB_LEFT : 0u) | (same(rx - 1, ry - 1) ? NB_ABOVE_LEFT : 0u) |
-               (same(rx, ry - 1) ? NB_ABOVE : 0u) | (same(rx + 1, ry - 1) ? NB_ABOVE_RIGHT : 0u);
-    }
-
-    // stage the CTU's tiles, TU records and residuals (packed in task order, one thread per
-    // TU) in one round of asynchronous copies
-    const int off = P.ictu_tu_off[idx], n_tu = P.ictu_tu_off[idx + 1] - off;
-    for (int i = tid; i < n_tu; i += IC_THREADS) {
-        cp_async16(&S.tu[i], &P.itu_rec[off + i]);
-        mbar_init1(&S.bar[i]);
-        S.itu_dep[i] = __ldg(&P.itu_dep[off + i]);
-    }
-    // the CTU's dependency entries are contiguous in task order
-    const uint32_t dfirst = __ldg(&P.itu_dep[off]) >> 6, dlast_e = __ldg(&P.itu_dep[off + n_tu - 1]);
-    const int n_dep = (int)((dlast_e >> 6) + (dlast_e & 63u)) - (int)dfirst;
-    const int staged = max(0, min(n_dep, IC_DEP_STAGE));
-    for (int q = tid; q < staged; q += IC_THREADS) S.dep[q] = __ldg(&P.dep_list[dfirst + q]);
-    const uint32_t wd = __ldg(&P.ictu_watch[idx]);
-    const int n_watch = min((int)(wd & 0xFFu), IC_MAX_WATCH);
-    for (int q = tid; q < n_watch; q += IC_THREADS) {
-        const uint32_t w = __ldg(&P.watch[(wd >> 8) + q]);
-        S.watch[q] = w;
-        if (w < (uint32_t)P.n_itu) cp_async16(&S.wtu[q], &P.itu_rec[w]);
-        mbar_init1(&S.bar[IC_MAX_TUS + q]);
-    }
-    // the CTU's origin in each plane's tile
-    auto origin = [&](int c) {
-        return c == 0 ? S.t_luma + IC_LP + IC_MARGIN : S.t_chroma[0] + (c - 1) * (IC_CH * IC_CP) + IC_CP + IC_MARGIN;
-    };
-    for (int c = 0; c < 3; c++) stage_tile(P, c, rx, ry, origin(c), tid, IC_THREADS);
-    for (int i = tid; i < n_tu; i += IC_THREADS) {
-        const int4 r = __ldg(&P.itu_res[off + i]);
-        for (int c = 0; c < r.z; c++) cp_async16(S.res + r.y + 8 * c, P.resid + r.x + 8 * c);
-    }
+    // Everything the CTU's tasks read, in one round of asynchronous copies: its tiles,
+    // residuals and plan.
+#pragma unroll 1
+    for (int q = tid; q < 2 * n_item; q += THREADS)
+        cp_async16(reinterpret_cast<uint4*>(S.task) + q, reinterpret_cast<const uint4*>(P.itu_task + c2.z) + q);
+#pragma unroll 1
+    for (int q = tid; q < 2 * n_watch; q += THREADS)
+        cp_async4(reinterpret_cast<uint32_t*>(S.watch) + q, reinterpret_cast<const uint32_t*>(P.watch_plan + c1.y) + q);
+    const int odd = c1.x & 1;   // rev goes in words
+#pragma unroll 1
+    for (int q = tid; q < (n_dep + odd + 1) / 2; q += THREADS)
+        cp_async4(S.rev + 2 * q, P.rev + c1.x - odd + 2 * q);
+    if (tid < IC_EDGES / 16) cp_async16(S.edge + 16 * tid, P.ictu_edge + S.ticket * IC_EDGES + 16 * tid);
+#pragma unroll 1
+    for (int q = tid; q < n_res / 8; q += THREADS) cp_async16(S.res + 8 * q, P.resid + c2.x + 8 * q);
+#pragma unroll 1
+    for (int c = 0; c < 3; c++) stage_tile<THREADS>(P, c, rx, ry, S.tiles + tile_origin(c), tid);
+    uint8_t* const rec = P.rec;
+    const int pitch_y = P.pitch_y, pitch_c = P.pitch_c, strong_intra = P.strong_intra;
+    uint64_t* const edge = P.edge;
     cp_async_wait_all();
     __syncthreads();
-
-    // what each TU reads, and the watched TUs that write some of it
-    const int ctbl = 1 << P.log2_ctb;
-    for (int i = tid; i < n_tu; i += IC_THREADS) {
-        const hevc_tu_t t = S.tu[i];
-        const int c = t.c_idx != 0;
-        const IntraAvail av = intra_avail(t.x, t.y, 1 << t.log2_size, P.width >> c, P.height >> c, P.log2_ctb - c, 1 + c,
-                                          S.nb);
-        const bool smooth = intra_smoothed(t.intra_mode, t.log2_size, c, P.intra_smoothing_disabled != 0);
-        const uint32_t need = intra_need(
-            intra_parts(t.intra_mode, t.log2_size, c, (t.flags & HEVC_TU_PCM) != 0, smooth), avail_segs(av));
-        S.av[i] = avail_pack(av, need);
-        const uint32_t dd = S.itu_dep[i];
-        for (int q = 0; q < (int)(dd & 63u); q++) {
-            const int at = (int)(dd >> 6) - (int)dfirst + q;
-            const uint32_t e = at >= 0 && at < staged ? S.dep[at] : __ldg(&P.dep_list[(dd >> 6) + q]);
-            const uint32_t j = e & INTRA_DEP_INDEX;
-            if ((e & INTRA_DEP_WATCH) && ((e >> INTRA_DEP_SEG_SHIFT) & need) && j < (uint32_t)n_watch)
-                atomicOr(&S.wneed[j / 32], 1u << (j % 32));
+#pragma unroll 1
+    for (int q = tid; q < n_item; q += THREADS) {
+        const IntraTask& k = S.task[q];
+        if (k.y0 == 0) {
+            mbar_init(&S.bar[k.bar], k.waits);
+            if (k.flags & TASK_STARTED) mbar_arrive(&S.bar[k.bar]);
         }
     }
+    if (tid < 16) S.res[IC_MAX_RES + tid] = 0;
+    if (tid == 32) S.tiles[IC_TILES] = 128;
     __syncthreads();
 
-    if (warp == IC_WORKERS) {
-        // The watcher: each lane follows the published completions of up to 4 watched TUs of
-        // other CTUs that some TU here reads from, all of them polled at once through L2
-        // (the wait is bounded like every other).  When some are seen, the warp copies
-        // each one's samples along this CTU into the tile's border and arrives on its
-        // watch barrier.  The acquire fence orders the other CTU's samples before the copies,
-        // the release arrival the copies before every read of a worker that waits on the
-        // barrier.
-        constexpr int R = IC_MAX_WATCH / 32;
-        bool pend[R], bad = false;
-        int32_t* flag[R];
+    // TU or watched TU s is complete: arrive at the TUs that wait for it, the first'th and every
+    // step'th after it
+    auto complete = [&](uint32_t source, int first, int step) {
+#pragma unroll 1
+        for (int q = first; q < (int)(source & 0xFFFFu); q += step) mbar_arrive(&S.bar[S.rev[odd + (source >> 16) + q]]);
+    };
+    if (warp == WARPS - 1) {
+        // The watcher: each lane follows up to 4 border words that TUs of other CTUs write and
+        // some TU here reads, all of them polled at once through L2 (the wait is bounded like
+        // every other).  A word that has come goes into the tile's border; with its last one
+        // a watched TU is complete.  The warp barrier and the release arrivals order the
+        // border's samples before every read of a TU that waits.
+        constexpr int R = IC_EDGES / 32;
+        const uint64_t* word[R];
+        uint8_t* to[R];       // where its 4 samples go
+        int step[R], slot[R]; // 1 along a row; the tile's pitch down the column
+        uint32_t pend = 0;
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            const int j = lane + 32 * r;
-            pend[r] = j < n_watch && ((S.wneed[r] >> lane) & 1u);
-            if (pend[r] && S.watch[j] >= (uint32_t)P.n_itu) bad = true;   // no such TU: refused
-            flag[r] = P.itu_done + (pend[r] && !bad ? S.watch[j] : 0);
-        }
-        if (__any_sync(0xffffffffu, bad)) {
-            if (bad) atomicOr(sticky, ST_BAD_RECORD);
-            S.abort = 1;
-            return;
+            const int l = lane + 32 * r;
+            slot[r] = S.edge[l];
+            const bool live = slot[r] < n_watch;
+            pend |= live ? 1u << r : 0u;
+            const int c = l < IC_EDGE_L ? 0 : (l < IC_EDGE_L + IC_EDGE_C ? 1 : 2);
+            const int i = l - (c == 0 ? 0 : IC_EDGE_L + (c - 1) * IC_EDGE_C), left0 = 1 + 2 * (c ? 8 : 16);
+            const int cw = (c ? ctbl / 2 : ctbl) / 4, tp = c ? IC_CP : IC_LP;
+            const bool column = i >= left0;
+            const int x4 = i - 1, y4 = i - left0;
+            const int from = column ? a - 1 : a - P.wctb + (x4 < 0 ? -1 : (x4 < cw ? 0 : 1));
+            const int at = column ? y4 : (x4 < 0 ? cw - 1 : (x4 < cw ? x4 : x4 - cw));
+            word[r] = edge + (live ? (int64_t)from * ctbl + edge_word(ctbl, c, column, at) : 0);
+            to[r] = S.tiles + tile_origin(c) + (column ? 4 * y4 * tp - 1 : 4 * x4 - tp);
+            step[r] = column ? tp : 1;
         }
         unsigned long long t0 = 0;
-        for (unsigned polls = 0;; polls++) {
-            int32_t v[R];
-            // relaxed polls (a GPU-scope acquire invalidates the SM's L1), one acquire fence
-            // once flags are seen
+        for (unsigned polls = 0; __any_sync(FULL, pend != 0u); polls++) {
+            uint64_t v[R];
 #pragma unroll
             for (int r = 0; r < R; r++) {
-                cuda::atomic_ref<int32_t, cuda::thread_scope_device> f(*flag[r]);
-                v[r] = pend[r] ? f.load(cuda::memory_order_relaxed) : epoch;
+                cuda::atomic_ref<const uint64_t, cuda::thread_scope_device> w(*word[r]);
+                v[r] = pend >> r & 1u ? w.load(cuda::memory_order_relaxed) : 0;
             }
-            uint32_t seen[R], some = 0, left = 0;
+            uint32_t seen = 0;
 #pragma unroll
-            for (int r = 0; r < R; r++) {
-                seen[r] = __ballot_sync(0xffffffffu, pend[r] && v[r] == epoch);
-                left |= __ballot_sync(0xffffffffu, pend[r] && v[r] != epoch);
-                some |= seen[r];
-            }
-            if (some) {
-                cuda::atomic_thread_fence(cuda::memory_order_acquire, cuda::thread_scope_device);
+            for (int r = 0; r < R; r++)
+                if ((pend >> r & 1u) && (int32_t)(v[r] >> 32) == epoch) {
+                    seen |= 1u << r;
+                    for (int b = 0; b < 4; b++) to[r][b * step[r]] = (uint8_t)(v[r] >> (8 * b));
+                }
+            pend &= ~seen;
+            if (__any_sync(FULL, seen != 0u)) {
                 __syncwarp();
 #pragma unroll
-                for (int r = 0; r < R; r++) {
-                    pend[r] = pend[r] && v[r] != epoch;
-                    for (uint32_t m = seen[r]; m; m &= m - 1u) {
-                        const int j = 32 * r + __ffs(m) - 1;
-                        const hevc_tu_t t = S.wtu[j];
-                        const int c = t.c_idx != 0, n = 1 << t.log2_size, ctbc = ctbl >> c;
-                        const int x = t.x - rx * ctbc, y = t.y - ry * ctbc;   // counted from this CTU
-                        const int pitch = c ? P.pitch_c : P.pitch_y, tp = c ? IC_CP : IC_LP;
-                        uint8_t* const o = origin(t.c_idx);
-                        const uint8_t* const src =
-                            P.rec + (t.c_idx == 0 ? 0 : (t.c_idx == 1 ? P.off_cb : P.off_cr)) + (int64_t)t.y * pitch + t.x;
-                        if (lane < n) {
-                            // its last row along this CTU's top, its last column along the left side
-                            if (y + n == 0 && x + lane >= -1 && x + lane < 2 * ctbc)
-                                o[x + lane - tp] = __ldcg(src + (int64_t)(n - 1) * pitch + lane);
-                            if (x + n == 0 && y + lane >= 0 && y + lane < ctbc)
-                                o[(y + lane) * tp - 1] = __ldcg(src + (int64_t)lane * pitch + n - 1);
-                        }
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&S.bar[IC_MAX_TUS + j]);
-                    }
-                }
+                for (int r = 0; r < R; r++)
+                    if ((seen >> r & 1u) && atomicSub(&S.watch[slot[r]].y, 1u) == 1u)
+                        complete(S.watch[slot[r]].x, 0, 1);
                 t0 = 0;
                 polls = 0;
+                continue;
             }
-            if (!left) break;
-            if (some) continue;
             cuda::atomic_ref<uint32_t, cuda::thread_scope_device> status(*sticky);
             const bool stop = !wait_goes_on(t0, polls, sticky, &S.abort) ||
                               (status.load(cuda::memory_order_relaxed) & ST_TIMEOUT);
-            if (__any_sync(0xffffffffu, stop)) {
+            if (__any_sync(FULL, stop)) {
                 S.abort = 1;
                 break;
             }
-            __nanosleep(32);
+            __nanosleep(20);
         }
         return;
     }
-    for (;;) {
-        int i = 0;
-        if (lane == 0) i = S.abort ? n_tu : atomicAdd(&S.next, 1);
-        i = __shfl_sync(0xffffffffu, i, 0);
-        if (i >= n_tu) break;
-        const hevc_tu_t tu = S.tu[i];
-        const uint32_t dd = S.itu_dep[i], av = S.av[i];
-        const int dcount = (int)(dd & 63u), doff = (int)(dd >> 6) - (int)dfirst;
-        const IntraWait wc{S.dep,  P.dep_list, S.bar, P.itu_done, sticky, &S.abort, (int)dfirst,   doff, dcount,
-                           staged, i,          n_watch, P.n_itu,  epoch,  lane,     avail_need(av)};
-        auto wait = [&]() -> bool { return intra_wait(wc); };
-        // after the warp barrier, lane 0's release arrival orders the warp's samples in the
-        // tile before the completion
-        auto done = [&]() {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&S.bar[i]);
-        };
-        const int ctbc = tu.c_idx ? ctbl / 2 : ctbl;
-        CtuTile tile;
-        tile.t = origin(tu.c_idx);
-        tile.pitch = tu.c_idx ? IC_CP : IC_LP;
-        tile.x0 = rx * ctbc;
-        tile.y0 = ry * ctbc;
-        const int16_t* res = (tu.flags & HEVC_TU_CODED) ? S.res + tu.coeff_offset : nullptr;
-        const bool ok = tu.log2_size == 2 ? intra_tu4(S.pic, tu, av, lane, tile, res, wait, done)
-                                          : intra_tu(S.pic, tu, av, lane, S.ws[warp], tile, res, wait, done);
-        if (!ok) {
-            if (lane == 0) S.abort = 1;
-            break;
-        }
-        if (tu.reserved[0] & ITU_PUBLISH) {
-            // the release store orders the warp's samples in the picture before the flag
-            __syncwarp();
-            if (lane == 0) {
-                cuda::atomic_ref<int32_t, cuda::thread_scope_device> g(P.itu_done[off + i]);
-                g.store(epoch, cuda::memory_order_release);
+    // Waits until all TUs that the TU of barrier `bar` waits for are complete; every lane acquires.
+    auto wait = [&](uint64_t* bar) {
+        unsigned long long t0 = 0;
+#pragma unroll 1
+        for (unsigned polls = 0;; polls++) {
+            // the lanes may see the barrier, the abort word or the clock at different moments
+            const bool over = mbar_try_wait0(bar);
+            if (__all_sync(FULL, over)) return true;
+            if (!__all_sync(FULL, over || wait_goes_on(t0, polls, sticky, &S.abort))) {
+                S.abort = 1;
+                return false;
             }
+        }
+    };
+    // Border words of rows y0 .. y0 + rows - 1 of a TU along the CTU's bottom and right.
+    auto publish = [&](const IntraTask& task, const uint8_t* t, int pitch, int y0, int rows, int n) {
+        uint64_t* const words = edge + (int64_t)a * ctbl + lane;
+        const uint64_t tag = (uint64_t)(uint32_t)epoch << 32;
+        if (task.row != TASK_NO_EDGE && y0 + rows == n && lane < n / 4) {
+            cuda::atomic_ref<uint64_t, cuda::thread_scope_device> w(words[task.row]);
+            w.store(tag | *reinterpret_cast<const uint32_t*>(t + (n - 1) * pitch + 4 * lane), cuda::memory_order_relaxed);
+        }
+        if (task.column != TASK_NO_EDGE && lane < rows / 4) {
+            const uint8_t* const col = t + (y0 + 4 * lane) * pitch + n - 1;
+            cuda::atomic_ref<uint64_t, cuda::thread_scope_device> w(words[task.column + y0 / 4]);
+            w.store(tag | (uint32_t)col[0] | (uint32_t)col[pitch] << 8 | (uint32_t)col[2 * pitch] << 16 |
+                        (uint32_t)col[3 * pitch] << 24,
+                    cuda::memory_order_relaxed);
+        }
+    };
+    uint32_t claim = claim_item(&S.next, lane);
+#pragma unroll 1
+    for (;;) {
+        const int item = (int)__shfl_sync(FULL, claim, 0);
+        if (item >= n_item) break;
+        // ---- before the wait: all that positions and the mode tell
+        const IntraTask task = S.task[item];
+        const bool chroma = task.flags & TASK_CHROMA;
+        const int pitch = chroma ? IC_CP : IC_LP, ppitch = chroma ? pitch_c : pitch_y;
+        uint8_t* const t = S.tiles + task.tile;   // the TU in its tile
+        const int count = (int)(task.source & 0xFFFFu);
+        // the first of the TUs that wait for this one, by lane
+        int next = lane < count ? S.rev[odd + (task.source >> 16) + lane] : -1;
+        if (task.log2 == 2) {
+            // 4x4 (most TUs, and most of a picture's dependency chain): one output sample per
+            // lane (the upper half of the warp repeats the lower), weighed from four samples of
+            // the tile (IntraTaps); lane k finds where index k of the reference array lies.
+            // No branch but DC's between the wait and the completion: one cost a lone warp
+            // some 25 cycles.
+            const uint2 taps = S.taps[(task.mode * 2 + (chroma ? 1 : 0)) * 16 + (lane & 15)];
+            const int w = task_where(task, 4, pitch, plan_min(lane, 16));
+            IntraTaps k = intra_taps_unpack(taps.x, taps.y);
+            int at[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) at[j] = __shfl_sync(FULL, w, k.i[j]);
+            int r = S.res[task.res + (lane & 15)];
+            const int x = lane & 3, y = (lane >> 2) & 3;
+            uint8_t* const to = t + y * pitch + x;
+            uint8_t* const pic = rec + (task.pic + (uint32_t)(y * ppitch + x));
+            // (keeps the compiler from moving this work behind the wait)
+#pragma unroll
+            for (int j = 0; j < 4; j++) asm volatile("" : "+r"(at[j]), "+r"(k.w[j]));
+            asm volatile("" : "+r"(k.add), "+r"(k.shift), "+r"(r), "+r"(next));
+            if (!wait(&S.bar[task.bar])) break;
+            claim = claim_item(&S.next, lane);   // the warp's next item: its latency hides here
+            int v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = t[at[j]];
+            if (task.mode == 1) v[1] = (int)(__reduce_add_sync(FULL, lane < 8 ? v[1] : 0) + 4) >> 3;   // predict_dc :295-317
+            const int p = clip_u8((v[0] * k.w[0] + v[1] * k.w[1] + v[2] * k.w[2] + v[3] * k.w[3] + k.add) >> k.shift);
+            const uint8_t out = (uint8_t)clip_u8(p + r);
+            if (lane < 16) *to = out;
+            // complete: after the warp barrier, each lane's release arrival orders the warp's
+            // samples in the tile before it
+            __syncwarp();
+            if (next >= 0) mbar_arrive(&S.bar[next]);
+            if (lane < 16) *pic = out;
+            if ((task.row & task.column) != TASK_NO_EDGE) publish(task, t, pitch, 0, 4, 4);
+            if (count > 32) complete(task.source, 32 + lane, 32);
+            continue;
+        }
+        // 8x8 and up.  Unsmoothed 8x8: two output samples per lane, (x, y) and (x, y + 4), in the
+        // same way.  Others: at[0] and at[1] samples lane and lane + 32 of the reference array
+        // in main order (mirrored for the horizontal modes), at[2] the last.
+        const int log2 = task.log2, n = 1 << log2, rows = plan_min(n, IC_BAND), y0 = task.y0;
+        const bool coded = task.flags & TASK_CODED, direct = log2 == 3 && !(task.flags & TASK_SMOOTH);
+        const int16_t* const res = S.res + (coded ? task.res : 0);
+        int at[4], at_b[4], r_a = 0, r_b = 0;
+        IntraTaps ka, kb;
+        if (direct) {
+            const int x = lane & 7, y = lane >> 3;
+            const int w = task_where(task, 8, pitch, lane), w32 = task_where(task, 8, pitch, 32);
+            const int mode = plan_min(task.mode, 34);
+            ka = intra_taps(3, mode, chroma, x, y, lane, task.angle, task.inv_angle);
+            kb = intra_taps(3, mode, chroma, x, y + 4, lane, task.angle, task.inv_angle);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int a32 = __shfl_sync(FULL, w, ka.i[j] & 31), b32 = __shfl_sync(FULL, w, kb.i[j] & 31);
+                at[j] = ka.i[j] == 32 ? w32 : a32;
+                at_b[j] = kb.i[j] == 32 ? w32 : b32;
+                if (task.mode == MODE_PCM) ka.w[j] = kb.w[j] = 0;
+                asm volatile("" : "+r"(at[j]), "+r"(at_b[j]), "+r"(ka.w[j]), "+r"(kb.w[j]));
+            }
+            if (task.mode == MODE_PCM) ka.add = kb.add = 0;
+            if (coded) {
+                r_a = res[lane];
+                r_b = res[lane + 32];
+            }
+        } else {
+            const bool vert = task.mode >= 18 || task.mode < 2;
+            at[0] = task_where(task, n, pitch, vert ? lane : 4 * n - lane);
+            at[1] = task_where(task, n, pitch, vert ? lane + 32 : 4 * n - lane - 32);
+            at[2] = task_where(task, n, pitch, vert ? 4 * n : 0);
+        }
+        if (!wait(&S.bar[task.bar])) break;
+        claim = claim_item(&S.next, lane);
+        if (direct) {
+            auto weigh = [&](const int (&v)[4], const IntraTaps& k, int r) {
+                return (uint8_t)clip_u8(
+                    clip_u8((v[0] * k.w[0] + v[1] * k.w[1] + v[2] * k.w[2] + v[3] * k.w[3] + k.add) >> k.shift) + r);
+            };
+            int v[4], u[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                v[j] = t[at[j]];
+                u[j] = t[at_b[j]];
+            }
+            if (task.mode == 1) v[1] = u[1] = (int)(__reduce_add_sync(FULL, lane < 16 ? v[1] : 0) + 8) >> 4;
+            uint8_t* const to = t + (lane >> 3) * pitch + (lane & 7);
+            to[0] = weigh(v, ka, r_a);
+            to[4 * pitch] = weigh(u, kb, r_b);
+        } else {
+            intra_predict(task, strong_intra, lane, S.ws[warp].ref, at[0], at[1], at[2], t, pitch, y0, rows, res, coded);
+        }
+        __syncwarp();
+        if (next >= 0) mbar_arrive(&S.bar[next]);
+        if (count > 32) complete(task.source, 32 + lane, 32);
+        if ((task.row & task.column) != TASK_NO_EDGE) publish(task, t, pitch, y0, rows, n);
+        // then the picture gets the band, off the chain
+#pragma unroll 1
+        for (int e = lane; e < rows * n / 4; e += 32) {
+            const int r = y0 + (e >> (log2 - 2)), c = 4 * (e & (n / 4 - 1));
+            *reinterpret_cast<uint32_t*>(rec + task.pic + r * ppitch + c) =
+                *reinterpret_cast<const uint32_t*>(t + r * pitch + c);
         }
     }
 }

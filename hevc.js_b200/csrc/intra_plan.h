@@ -1,7 +1,8 @@
 // intra_plan.h — what an intra TU reads, from positions and its mode alone: which of its
 // reference samples are available (build_reference_samples, intra_prediction.cpp:102-133),
 // which sample stands in for one that is not (:177-197), which parts of the reference array
-// the prediction reads, and for a 4x4 TU the samples and weights of each output sample
+// the prediction reads, and for a 4x4 or 8x8 TU the samples and weights of each output
+// sample
 // (:263-422).  k_intra_ctus works all of it out before it waits for any sample.  Host and
 // device code; no CUDA header is needed, so the rules are tested on the CPU.
 #pragma once
@@ -9,9 +10,9 @@
 #include <cstdint>
 
 #ifdef __CUDACC__
-#define HEVC_HD __host__ __device__ __forceinline__
+#define HEVC_HD constexpr __host__ __device__ __forceinline__
 #else
-#define HEVC_HD inline
+#define HEVC_HD constexpr inline
 #endif
 
 namespace hevcgpu {
@@ -59,7 +60,7 @@ struct IntraAvail {
 HEVC_HD IntraAvail intra_avail(int x, int y, int n, int pw, int ph, int log2c, int sub, uint32_t nb) {
     const int cs = 1 << log2c, xi = x & (cs - 1), yi = y & (cs - 1);
     const uint32_t z = zorder16((uint32_t)(xi * sub) >> 2, (uint32_t)(yi * sub) >> 2);
-    IntraAvail a;
+    IntraAvail a{};
     a.n = n;
     a.l = x > 0 && (xi > 0 || (nb & NB_LEFT));
     a.t = y > 0 && (yi > 0 || (nb & NB_ABOVE));
@@ -67,7 +68,7 @@ HEVC_HD IntraAvail intra_avail(int x, int y, int n, int pw, int ph, int log2c, i
     const bool bl = a.l && yi + n < cs &&
                     (xi == 0 || zorder16((uint32_t)((xi - 1) * sub) >> 2, (uint32_t)((yi + n) * sub) >> 2) < z);
     a.bl = bl ? plan_max(0, plan_min(n, ph - (y + n))) : 0;
-    bool tr;
+    bool tr = false;
     if (yi > 0) tr = xi + n < cs && zorder16((uint32_t)((xi + n) * sub) >> 2, (uint32_t)((yi - 1) * sub) >> 2) < z;
     else tr = y > 0 && (nb & (xi + n < cs ? NB_ABOVE : NB_ABOVE_RIGHT));
     a.tr = tr ? plan_max(0, plan_min(n, pw - (x + n))) : 0;
@@ -78,16 +79,14 @@ HEVC_HD uint32_t avail_segs(const IntraAvail& a) {
     return (a.bl ? SEG_BL : 0u) | (a.l ? SEG_L : 0u) | (a.c ? SEG_C : 0u) | (a.t ? SEG_T : 0u) | (a.tr ? SEG_TR : 0u);
 }
 
-// Packed form (bits 0-5 bl, 6-11 tr, 12 l, 13 c, 14 t; 16-20 the parts the TU reads).
-HEVC_HD uint32_t avail_pack(const IntraAvail& a, uint32_t need) {
-    return (uint32_t)a.bl | ((uint32_t)a.tr << 6) | ((uint32_t)a.l << 12) | ((uint32_t)a.c << 13) |
-           ((uint32_t)a.t << 14) | (need << 16);
+// Packed form: bits 0-5 bl, 6-11 tr, 12 l, 13 c, 14 t.
+HEVC_HD uint32_t avail_pack(const IntraAvail& a) {
+    return (uint32_t)a.bl | ((uint32_t)a.tr << 6) | ((uint32_t)a.l << 12) | ((uint32_t)a.c << 13) | ((uint32_t)a.t << 14);
 }
 HEVC_HD IntraAvail avail_unpack(uint32_t w, int n) {
     return IntraAvail{n, (int)(w & 63u), (int)((w >> 6) & 63u), ((w >> 12) & 1u) != 0, ((w >> 13) & 1u) != 0,
                       ((w >> 14) & 1u) != 0};
 }
-HEVC_HD uint32_t avail_need(uint32_t w) { return (w >> 16) & SEG_ALL; }
 
 // The index whose sample stands at index i: i itself when available, else the nearest
 // available one below it, else the first available one (:177-197); -1 when none is.
@@ -150,6 +149,31 @@ HEVC_HD uint32_t intra_need(uint32_t parts, uint32_t avail) {
     return need;
 }
 
+// intraPredAngle and invAngle of the angular modes (intra_prediction.cpp:263-422).
+HEVC_HD int intra_angle(int mode) {
+    constexpr int8_t t[35] = {0,   0,   32,  26,  21,  17,  13,  9,   5,  2,  0,  -2, -5, -9, -13, -17, -21, -26,
+                              -32, -26, -21, -17, -13, -9,  -5,  -2,  0,  2,  5,  9,  13, 17, 21,  26,  32};
+    return t[mode];
+}
+HEVC_HD int intra_inv_angle(int mode) {
+    constexpr int16_t t[35] = {0,    0,   256, 315, 390, 482, 630, 910, 1638, 4096, 0,    4096, 1638, 910, 630, 482, 390, 315,
+                               256,  315, 390, 482, 630, 910, 1638, 4096, 0,  4096, 1638, 910,  630,  482, 390, 315, 256};
+    return t[mode];
+}
+
+struct IntraAngles {
+    int8_t angle[35];
+    int16_t inv[35];
+};
+HEVC_HD IntraAngles intra_angles() {
+    IntraAngles r{};
+    for (int mode = 0; mode < 35; mode++) {
+        r.angle[mode] = (int8_t)intra_angle(mode);
+        r.inv[mode] = (int16_t)intra_inv_angle(mode);
+    }
+    return r;
+}
+
 // Main reference entry q of an angular mode as a reference array index: q >= 0 runs along
 // the main side, q < 0 is the side reference projected through invAngle (:346-368).  Entries
 // past the end are read only with weight 0.
@@ -158,32 +182,64 @@ HEVC_HD int intra_main_index(bool vert, int inv, int n, int q) {
     return plan_max(0, plan_min(4 * n, vert ? 2 * n + k : 2 * n - k));
 }
 
-// The prediction of sample (x, y) of a 4x4 TU as one form over four samples of the
-// (substituted) reference array:
+// The prediction of sample (x, y) of an unsmoothed 4x4 or 8x8 TU as one form over four samples
+// of the (substituted) reference array:
 //   clip((i[0] * w[0] + i[1] * w[1] + i[2] * w[2] + i[3] * w[3] + add) >> shift)
 // covers planar (:263-289), angular (:323-422) and the boundary filters of modes 26 and 10
 // (p + ((side - corner) >> 1) = (2p + side - corner) >> 1).  DC (:295-317): i[1] is one of
-// the 8 samples of the sum, by `lane`, and the rounded mean takes its place.
-struct IntraTaps4 {
+// the 2n samples of the sum, by `lane`, and the rounded mean takes its place.
+struct IntraTaps {
     int i[4], w[4], add, shift;
 };
-HEVC_HD IntraTaps4 intra_taps4(int mode, bool chroma, int x, int y, int lane, int ang, int inv) {
-    if (mode == 0) return IntraTaps4{{7 - y, 13, 9 + x, 3}, {3 - x, x + 1, 3 - y, y + 1}, 4, 3};
+HEVC_HD IntraTaps intra_taps(int log2, int mode, bool chroma, int x, int y, int lane, int ang, int inv) {
+    const int n = 1 << log2;
+    if (mode == 0)
+        return IntraTaps{{2 * n - 1 - y, 3 * n + 1, 2 * n + 1 + x, n - 1}, {n - 1 - x, x + 1, n - 1 - y, y + 1}, n, log2 + 1};
     if (mode == 1) {
         const bool ex = !chroma && x == 0, ey = !chroma && y == 0;
-        const int k = lane & 7;
-        return IntraTaps4{{9 + x, k < 4 ? 4 + k : 5 + k, 7 - y, 8},
-                          {ey ? 1 : 0, 4 - (ex ? 1 : 0) - (ey ? 1 : 0), ex ? 1 : 0, 0},
-                          ex || ey ? 2 : 0,
-                          2};
+        const int k = lane & (2 * n - 1);
+        return IntraTaps{{2 * n + 1 + x, k < n ? n + k : n + 1 + k, 2 * n - 1 - y, 2 * n},
+                         {ey ? 1 : 0, 4 - (ex ? 1 : 0) - (ey ? 1 : 0), ex ? 1 : 0, 0},
+                         ex || ey ? 2 : 0,
+                         2};
     }
     const bool vert = mode >= 18;
     const int along = vert ? y : x, across = vert ? x : y;
     const int idx = ((along + 1) * ang) >> 5, fr = ((along + 1) * ang) & 31, q = across + 1 + idx;
-    const int a = intra_main_index(vert, inv, 4, q), b = intra_main_index(vert, inv, 4, q + 1);
-    const int side = vert ? 7 - along : 9 + along;
-    if (ang == 0 && !chroma && across == 0) return IntraTaps4{{a, b, side, 8}, {2, 0, 1, -1}, 0, 1};
-    return IntraTaps4{{a, b, side, 8}, {32 - fr, fr, 0, 0}, 16, 5};
+    const int a = intra_main_index(vert, inv, n, q), b = intra_main_index(vert, inv, n, q + 1);
+    const int side = vert ? 2 * n - 1 - along : 2 * n + 1 + along;
+    if (ang == 0 && !chroma && across == 0) return IntraTaps{{a, b, side, 2 * n}, {2, 0, 1, -1}, 0, 1};
+    return IntraTaps{{a, b, side, 2 * n}, {32 - fr, fr, 0, 0}, 16, 5};
+}
+
+// The taps of every mode, plane kind and lane of a 4x4 TU, 8 bytes each: word 0 the four
+// indices (5 bits each), w[0] and w[1] (6 bits each); word 1 w[2] (bits 0-2), w[3] + 1 (3-5),
+// add (6-10), shift (11-13).  "Mode" MODE_PCM predicts nothing (weights 0): a PCM TU's samples
+// are its levels.
+constexpr int MODE_PCM = 35;
+struct IntraTapTable {
+    uint32_t t[36][2][16][2];
+};
+HEVC_HD IntraTapTable intra_tap_table() {
+    IntraTapTable r{};
+    for (int i = 0; i < 32; i++) r.t[MODE_PCM][i / 16][i % 16][1] = 1u << 3;
+    for (int mode = 0; mode < 35; mode++)
+        for (int c = 0; c < 2; c++)
+            for (int lane = 0; lane < 16; lane++) {
+                const IntraTaps k = intra_taps(2, mode, c != 0, lane & 3, lane >> 2, lane, intra_angle(mode),
+                                               intra_inv_angle(mode));
+                r.t[mode][c][lane][0] = (uint32_t)k.i[0] | (uint32_t)k.i[1] << 5 | (uint32_t)k.i[2] << 10 |
+                                        (uint32_t)k.i[3] << 15 | (uint32_t)k.w[0] << 20 | (uint32_t)k.w[1] << 26;
+                r.t[mode][c][lane][1] =
+                    (uint32_t)k.w[2] | (uint32_t)(k.w[3] + 1) << 3 | (uint32_t)k.add << 6 | (uint32_t)k.shift << 11;
+            }
+    return r;
+}
+HEVC_HD IntraTaps intra_taps_unpack(uint32_t a, uint32_t b) {
+    return IntraTaps{{(int)(a & 31u), (int)(a >> 5 & 31u), (int)(a >> 10 & 31u), (int)(a >> 15 & 31u)},
+                      {(int)(a >> 20 & 63u), (int)(a >> 26), (int)(b & 7u), (int)(b >> 3 & 7u) - 1},
+                      (int)(b >> 6 & 31u),
+                      (int)(b >> 11)};
 }
 
 }  // namespace hevcgpu

@@ -138,14 +138,18 @@ __global__ void __launch_bounds__(128) k_residual(const __grid_constant__ SegTab
     const int item = (blockIdx.x - sg.block0) * TUS + slot;
     const bool live = item < sg.n_items;
     const PicDesc& P = *sg.pic;
-    hevc_tu_t t = live ? P.tus[static_cast<const int32_t*>(sg.items)[item]] : hevc_tu_t{};
+    const uint32_t id = live ? static_cast<const uint32_t*>(sg.items)[item] : 0u;
+    const bool intra_item = (id & RES_INTRA_ITEM) != 0;   // residual into resid, for the intra stage
+    const uint32_t at = id & ~RES_INTRA_ITEM;
+    hevc_tu_t t = live ? (intra_item ? P.itu_rec[at] : P.tus[at]) : hevc_tu_t{};
+    const int2 from_to = intra_item ? P.itu_res[at] : make_int2((int)t.coeff_offset, 0);
     const bool bypass = t.flags & (HEVC_TU_BYPASS | HEVC_TU_PCM);   // levels are the residual
     const bool tskip = (t.flags & HEVC_TU_TSKIP) && !bypass;
     const bool dst4 = (LOG2 == 2) && (t.flags & HEVC_TU_INTRA) && t.c_idx == 0;
 
     // load row j of the levels and dequantise it
     if (live) {
-        const int16_t* src = P.coeffs + t.coeff_offset + j * N;
+        const int16_t* src = P.coeffs + (uint32_t)from_to.x + j * N;
         int16_t v[N];
         if constexpr (N >= 8) {
 #pragma unroll
@@ -203,11 +207,20 @@ __global__ void __launch_bounds__(128) k_residual(const __grid_constant__ SegTab
         for (int k = 0; k < N; k++) r[k] = clip3(-32768, 32767, (d[k] + 2048) >> 12);
     }
 
-    if (mode == RES_PICTURE && (t.flags & HEVC_TU_INTRA)) {
-        // residual of an intra TU: the wavefront adds it to its prediction
-        int16_t* dst = P.resid + t.coeff_offset + j * N;
+    if (intra_item) {
+        // residual of an intra TU: the wavefront adds it to its prediction.  A row goes out in
+        // 16-byte words (8-byte ones for 4x4): residuals lie at multiples of 16 samples
+        uint32_t w[N / 2];
 #pragma unroll
-        for (int k = 0; k < N; k++) dst[k] = (int16_t)r[k];
+        for (int k = 0; k < N / 2; k++) w[k] = __byte_perm((uint32_t)r[2 * k], (uint32_t)r[2 * k + 1], 0x5410);
+        int16_t* dst = P.resid + from_to.y + j * N;
+        if constexpr (N >= 8) {
+#pragma unroll
+            for (int q = 0; q < N / 8; q++)
+                reinterpret_cast<uint4*>(dst)[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+        } else {
+            *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+        }
         return;
     }
     const uint8_t* pred;

@@ -65,15 +65,6 @@ __device__ __forceinline__ int dp2a_hi(uint32_t a, uint32_t b, int c) {
     asm("dp2a.hi.s32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
-// v0..v3 saturated to 0..255 and packed as bytes 0..3 (PTX cvt.pack.sat: the low 16 bits
-// of c move up by 16 and a, b take bits 15..8 and 7..0).
-__device__ __forceinline__ uint32_t pack_sat_u8x4(int v0, int v1, int v2, int v3) {
-    uint32_t t, d;
-    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, 0;" : "=r"(t) : "r"(v3), "r"(v2));
-    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(v1), "r"(v0), "r"(t));
-    return d;
-}
-
 // Strip work item, 32 bits: PU index (bits 0-19), strip column / 4 (20-23), strip row / 16
 // (24-25), rows code (26-28: luma rows / 4 - 1, chroma rows / 2 - 1), chroma plane (29:
 // 0 Cb, 1 Cr).  Offsets and rows are in samples of the strip's plane.

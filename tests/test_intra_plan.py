@@ -1,7 +1,7 @@
 """intra_plan.h (what an intra TU reads, worked out from positions and its mode) against
 per-sample definitions of its own, on the CPU: availability and substitution sample by sample
 (intra_prediction.cpp:102-133, 177-197), the parts of the reference array a mode reads against
-the samples its formulas touch, and the 4x4 weights against the prediction formulas
+the samples its formulas touch, and the 4x4 and 8x8 weights against the prediction formulas
 (:263-422).  All results are integers: equality."""
 import ctypes as C
 import os
@@ -20,21 +20,22 @@ WRAPPER = r"""
 using namespace hevcgpu;
 extern "C" {
 void subst(int x, int y, int n, int pw, int ph, int log2c, int sub, unsigned nb, int* out) {
-    const unsigned w = avail_pack(intra_avail(x, y, n, pw, ph, log2c, sub, nb), 0);
+    const unsigned w = avail_pack(intra_avail(x, y, n, pw, ph, log2c, sub, nb));
     for (int i = 0; i <= 4 * n; i++) out[i] = intra_substitute(avail_unpack(w, n), i);
 }
 int smoothed(int mode, int log2, int chroma, int disabled) { return intra_smoothed(mode, log2, chroma, disabled); }
 unsigned need(int mode, int log2, int chroma, int pcm, int smooth, int bl, int tr, int l, int c, int t) {
     const IntraAvail a{1 << log2, bl, tr, l != 0, c != 0, t != 0};
-    const unsigned w = avail_pack(a, intra_need(intra_parts(mode, log2, chroma, pcm, smooth), avail_segs(a)));
-    return avail_need(w);
+    return intra_need(intra_parts(mode, log2, chroma, pcm, smooth), avail_segs(a));
 }
 int substitute(int log2, int bl, int tr, int l, int c, int t, int i) {
     return intra_substitute(IntraAvail{1 << log2, bl, tr, l != 0, c != 0, t != 0}, i);
 }
 int main_index(int vert, int inv, int n, int q) { return intra_main_index(vert, inv, n, q); }
-void taps4(int mode, int chroma, int x, int y, int lane, int ang, int inv, int* out) {
-    const IntraTaps4 k = intra_taps4(mode, chroma, x, y, lane, ang, inv);
+void taps(int log2, int mode, int chroma, int x, int y, int lane, int* out) {
+    static const IntraTapTable table = intra_tap_table();
+    const IntraTaps k = log2 == 2 ? intra_taps_unpack(table.t[mode][chroma][lane][0], table.t[mode][chroma][lane][1])
+                                  : intra_taps(log2, mode, chroma, x, y, lane, intra_angle(mode), intra_inv_angle(mode));
     for (int j = 0; j < 4; j++) { out[j] = k.i[j]; out[4 + j] = k.w[j]; }
     out[8] = k.add;
     out[9] = k.shift;
@@ -152,47 +153,50 @@ def test_needed_parts_hold_every_sample_read(plan, log2):
 
 @pytest.mark.parametrize("mode", range(35))
 @pytest.mark.parametrize("chroma", [0, 1])
-def test_taps_of_a_4x4_block_are_its_prediction(plan, mode, chroma):
+@pytest.mark.parametrize("log2", [2, 3])
+def test_taps_of_a_block_are_its_prediction(plan, mode, chroma, log2):
     rng = random.Random(mode)
-    for trial in range(24):
-        R = [rng.choice((0, 255)) if trial < 8 else rng.randrange(256) for _ in range(17)]
-        dc = (sum(R[4:8]) + sum(R[9:13]) + 4) >> 3
-        for lane in range(16):
-            x, y = lane & 3, lane >> 2
-            left, top, corner = R[7 - y], R[9 + x], R[8]
-            if mode == 0:
-                want = ((3 - x) * left + (x + 1) * R[13] + (3 - y) * top + (y + 1) * R[3] + 4) >> 3
-            elif mode == 1:
-                want = dc
-                if not chroma and x == 0 and y == 0:
-                    want = (left + 2 * dc + top + 2) >> 2
-                elif not chroma and y == 0:
-                    want = (top + 3 * dc + 2) >> 2
-                elif not chroma and x == 0:
-                    want = (left + 3 * dc + 2) >> 2
-            else:
-                vert = mode >= 18
-                main = (lambda q: R[8 + q] if vert else R[8 - q])
-                side = (lambda k: R[8 - k] if vert else R[8 + k])
-                ref = (lambda q: main(q) if q >= 0 else side(min(8, (-q * INV[mode] + 128) >> 8)))
-                along, across = (y, x) if vert else (x, y)
-                idx, fr = (along + 1) * ANGLE[mode] >> 5, (along + 1) * ANGLE[mode] & 31
-                want = ref(across + 1 + idx)
-                if fr:
-                    want = ((32 - fr) * want + fr * ref(across + 2 + idx) + 16) >> 5
-                if not chroma and mode == 26 and x == 0:
-                    want = min(255, max(0, want + ((left - corner) >> 1)))
-                if not chroma and mode == 10 and y == 0:
-                    want = min(255, max(0, want + ((top - corner) >> 1)))
-            k = (C.c_int * 10)()
-            plan.taps4(mode, chroma, x, y, lane, ANGLE[mode], INV[mode], k)
-            v = [R[k[j]] for j in range(4)]
-            if mode == 1:
-                total = 0
-                for other in range(8):
-                    k2 = (C.c_int * 10)()
-                    plan.taps4(mode, chroma, x, y, other, 0, 0, k2)
-                    total += R[k2[1]]
-                v[1] = (total + 4) >> 3
-            got = sum(v[j] * k[4 + j] for j in range(4)) + k[8] >> k[9]
-            assert min(255, max(0, got)) == want, (lane, trial)
+    n = 1 << log2
+    for trial in range(24 if log2 == 2 else 6):
+        R = [rng.choice((0, 255)) if trial < 2 * n else rng.randrange(256) for _ in range(4 * n + 1)]
+        dc = (sum(R[n:2 * n]) + sum(R[2 * n + 1:3 * n + 1]) + n) >> (log2 + 1)
+        for y in range(n):
+            for x in range(n):
+                left, top, corner = R[2 * n - 1 - y], R[2 * n + 1 + x], R[2 * n]
+                if mode == 0:
+                    want = ((n - 1 - x) * left + (x + 1) * R[3 * n + 1] + (n - 1 - y) * top + (y + 1) * R[n - 1] + n) >> \
+                        (log2 + 1)
+                elif mode == 1:
+                    want = dc
+                    if not chroma and x == 0 and y == 0:
+                        want = (left + 2 * dc + top + 2) >> 2
+                    elif not chroma and y == 0:
+                        want = (top + 3 * dc + 2) >> 2
+                    elif not chroma and x == 0:
+                        want = (left + 3 * dc + 2) >> 2
+                else:
+                    vert = mode >= 18
+                    main = (lambda q: R[2 * n + q] if vert else R[2 * n - q])
+                    side = (lambda k: R[2 * n - k] if vert else R[2 * n + k])
+                    ref = (lambda q: main(q) if q >= 0 else side(min(2 * n, (-q * INV[mode] + 128) >> 8)))
+                    along, across = (y, x) if vert else (x, y)
+                    idx, fr = (along + 1) * ANGLE[mode] >> 5, (along + 1) * ANGLE[mode] & 31
+                    want = ref(across + 1 + idx)
+                    if fr:
+                        want = ((32 - fr) * want + fr * ref(across + 2 + idx) + 16) >> 5
+                    if not chroma and mode == 26 and x == 0:
+                        want = min(255, max(0, want + ((left - corner) >> 1)))
+                    if not chroma and mode == 10 and y == 0:
+                        want = min(255, max(0, want + ((top - corner) >> 1)))
+                k = (C.c_int * 10)()
+                plan.taps(log2, mode, chroma, x, y, y * n + x, k)
+                v = [R[k[j]] for j in range(4)]
+                if mode == 1:
+                    total = 0
+                    for other in range(2 * n):
+                        k2 = (C.c_int * 10)()
+                        plan.taps(log2, mode, chroma, x, y, other, k2)
+                        total += R[k2[1]]
+                    v[1] = (total + n) >> (log2 + 1)
+                got = sum(v[j] * k[4 + j] for j in range(4)) + k[8] >> k[9]
+                assert min(255, max(0, got)) == want, (x, y, trial)
