@@ -1281,6 +1281,11 @@ struct Launcher {
     hevcgpu_ctx* ctx;
     cudaStream_t s;
 
+    // Launches after the first of a sequence may start before the one before has ended
+    // (pdl_next / pdl_wait in the kernels).  Anything else queued between two of them (a copy,
+    // a memset, an event) makes the later one wait for all before it, as usual.
+    bool first = true;
+
     template <typename K, typename... A>
     int go(K kernel, dim3 grid, dim3 block, A... args) {
         return go_smem(kernel, grid, block, 0, args...);
@@ -1288,9 +1293,23 @@ struct Launcher {
     template <typename K, typename... A>
     int go_smem(K kernel, dim3 grid, dim3 block, size_t smem, A... args) {
         if (grid.x == 0 || grid.y == 0 || grid.z == 0) return HEVCGPU_OK;
-        kernel<<<grid, block, smem, s>>>(args...);
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid;
+        cfg.blockDim = block;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cfg.attrs = &attr;
+        cfg.numAttrs = first ? 0 : 1;
+        first = false;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return fail(HEVCGPU_ECUDA, "kernel launch: %s", cudaGetErrorString(e));
+        }
         ctx->launches++;
-        CUDA_TRY(cudaGetLastError());
         return HEVCGPU_OK;
     }
 
@@ -1380,9 +1399,61 @@ bool intra_wide(int ctus, int64_t items, int depth, int sms) {
     return items >= 16ll * ctus && (items >= 64ll * ctus || 400ll * depth >= items * 163 / sms);
 }
 
+// The intra launches of a batch, one per group of up to MAX_SEGS pictures: CTAs take intra CTUs
+// by ticket in wavefront order per picture; block0 = intra CTUs of earlier pictures, aux1 =
+// epoch.
+struct IntraLaunch {
+    SegTable t;
+    int total;
+    bool wide;
+};
+int intra_launches(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n, std::vector<IntraLaunch>& out) {
+    for (int k = 0; k < n;) {
+        IntraLaunch g;
+        std::memset(&g.t, 0, sizeof(g.t));
+        int total = 0, depth = 0;
+        int64_t items = 0;
+        for (; k < n && g.t.n < MAX_SEGS; k++) {
+            hevcgpu_job* j = jobs[k];
+            if (j->n_ictu == 0) continue;
+            Seg& sg = g.t.s[g.t.n++];
+            sg.pic = static_cast<const PicDesc*>(j->desc.p);
+            sg.items = j->d_ictu;
+            sg.block0 = total;
+            // border words hold the epoch of the launch that wrote them; restart the epochs
+            // from zero words before they would reach the sign bit
+            if (j->epoch >= 0x7FFFFFF0) {
+                CUDA_TRY(cudaMemsetAsync(j->host_desc.edge, 0, j->edge_bytes, ex.stream));
+                j->epoch = 0;
+            }
+            sg.aux1 = ++j->epoch;
+            total += j->n_ictu;
+            items += j->n_items;
+            depth = std::max(depth, j->depth);
+        }
+        if (g.t.n == 0) continue;
+        g.total = total;
+        g.wide = intra_wide(total, items, depth, ctx->sm_count);
+        out.push_back(g);
+    }
+    return HEVCGPU_OK;
+}
+
 int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n, int stages, int res_mode) {
     Launcher L{ctx, ex.stream};
     int rc;
+    // the intra stage's plan comes first: it needs only the records (those of later groups
+    // follow the group before, whose tickets they use again)
+    std::vector<IntraLaunch> intra;
+    uint32_t* sticky = reinterpret_cast<uint32_t*>(static_cast<FlowState*>(ex.flow) + 1);
+    auto plan = [&](const IntraLaunch& g, bool later) {
+        return L.go(k_intra_plan, dim3(g.total), dim3(IP_THREADS), g.t, ex.tickets(), (int)later, sticky);
+    };
+    if ((stages & ST_INTRA) && (rc = intra_launches(ctx, ex, jobs, n, intra))) return rc;
+    if (!intra.empty()) {
+        StageMark m(ctx, ex.stream, 3);
+        if ((rc = plan(intra[0], false))) return rc;
+    }
     if ((stages & ST_DEBLOCK) && !(stages & ST_MC)) {   // with MC, its luma strips write the grid
         StageMark m(ctx, ex.stream, 0);
         rc = L.pictures(k_motion_grid, jobs, n, 256, 1, [](hevcgpu_job* j) { return (j->n_pus * 32 + 255) / 256; });
@@ -1414,49 +1485,14 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
             if (rc) return rc;
         }
     }
-    if (stages & ST_INTRA) {
+    for (const IntraLaunch& g : intra) {
         StageMark m(ctx, ex.stream, 3);
-        // one launch per group of up to MAX_SEGS pictures: CTAs take intra CTUs by ticket
-        // in wavefront order per picture; block0 = intra CTUs of earlier pictures, aux1 = epoch
-        int k = 0;
-        while (k < n) {
-            SegTable t;
-            std::memset(&t, 0, sizeof(t));
-            int total = 0;
-            int64_t items = 0;
-            int depth = 0;
-            for (; k < n && t.n < MAX_SEGS; k++) {
-                hevcgpu_job* j = jobs[k];
-                if (j->n_ictu == 0) continue;
-                Seg& sg = t.s[t.n++];
-                sg.pic = static_cast<const PicDesc*>(j->desc.p);
-                sg.block0 = total;
-                sg.items = j->d_ictu;
-                // border words hold the epoch of the launch that wrote them; restart the epochs
-                // from zero words before they would reach the sign bit
-                if (j->epoch >= 0x7FFFFFF0) {
-                    CUDA_TRY(cudaMemsetAsync(j->host_desc.edge, 0, j->edge_bytes, ex.stream));
-                    j->epoch = 0;
-                }
-                sg.aux1 = ++j->epoch;
-                total += j->n_ictu;
-                items += j->n_items;
-                depth = std::max(depth, j->depth);
-            }
-            if (t.n == 0) continue;
-            FlowState* fs = static_cast<FlowState*>(ex.flow);
-            uint32_t* sticky = reinterpret_cast<uint32_t*>(fs + 1);
-            int32_t* tickets = ex.tickets();
-            CUDA_TRY(cudaMemsetAsync(tickets, 0, sizeof(int32_t) * (size_t)t.n, ex.stream));
-            rc = L.go(k_intra_plan, dim3(total), dim3(IP_THREADS), t, sticky);
-            if (rc) return rc;
-            const bool wide = intra_wide(total, items, depth, ctx->sm_count);
-            rc = wide ? L.go_smem(k_intra_ctus<IC_WIDE>, dim3(total), dim3(32 * IC_WIDE), sizeof(IntraSmem), t, tickets,
-                                  total, sticky)
-                      : L.go_smem(k_intra_ctus<IC_NARROW>, dim3(total), dim3(32 * IC_NARROW), sizeof(IntraSmem), t,
-                                  tickets, total, sticky);
-            if (rc) return rc;
-        }
+        if (&g != &intra[0] && (rc = plan(g, true))) return rc;
+        rc = g.wide ? L.go_smem(k_intra_ctus<IC_WIDE>, dim3(g.total), dim3(32 * IC_WIDE), sizeof(IntraSmem), g.t, ex.tickets(),
+                                g.total, sticky)
+                    : L.go_smem(k_intra_ctus<IC_NARROW>, dim3(g.total), dim3(32 * IC_NARROW), sizeof(IntraSmem), g.t,
+                                ex.tickets(), g.total, sticky);
+        if (rc) return rc;
     }
     if (stages & ST_DEBLOCK) {
         {

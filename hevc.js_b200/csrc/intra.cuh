@@ -389,10 +389,14 @@ constexpr int AV_NEED_SHIFT = 23;            // bits 23-27 the parts of its refe
 constexpr int AV_BANDS_SHIFT = 28;           // bits 28-30 its bands
 constexpr int IP_THREADS = 128;
 
-__global__ void __launch_bounds__(IP_THREADS) k_intra_plan(const __grid_constant__ SegTable st, uint32_t* sticky) {
+__global__ void __launch_bounds__(IP_THREADS) k_intra_plan(const __grid_constant__ SegTable st, int32_t* tickets,
+                                                             int later, uint32_t* sticky) {
     __shared__ uint32_t s_av[IC_MAX_TUS], s_count[IC_SOURCES], s_fill[IC_SOURCES], s_total, s_bad;
     __shared__ uint8_t s_edge[IC_EDGES];
     const int tid = threadIdx.x, lane = tid % 32;
+    pdl_next();   // MC and the residuals' transforms need nothing of the plan
+    if (later) pdl_wait();   // the tickets are in use by the group before
+    if (blockIdx.x == 0 && tid < st.n) tickets[tid] = 0;
     const int k = find_seg(st, blockIdx.x);
     const PicDesc& P = *st.s[k].pic;
     const int idx = blockIdx.x - st.s[k].block0;
@@ -521,6 +525,7 @@ __global__ void __launch_bounds__(IP_THREADS) k_intra_plan(const __grid_constant
     if (tid < IC_EDGES / 4)
         reinterpret_cast<uint32_t*>(P.ictu_edge)[idx * (IC_EDGES / 4) + tid] = reinterpret_cast<const uint32_t*>(s_edge)[tid];
     if (tid == 0 && s_bad) atomicOr(sticky, ST_BAD_RECORD);   // k_intra_ctus then does nothing
+    pdl_wait();
 }
 
 // ---------------------------------------------------------------------------------------
@@ -551,6 +556,11 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS + (WARPS > 8)) k_intra_
     extern __shared__ __align__(16) uint8_t smem_raw[];
     IntraSmem& S = *reinterpret_cast<IntraSmem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
+    pdl_next();
+#pragma unroll 1
+    for (int q = tid; q < (int)sizeof(S.taps) / 16; q += THREADS)
+        cp_async16(reinterpret_cast<uint4*>(S.taps) + q, reinterpret_cast<const uint4*>(c_intra_taps.t) + q);
+    pdl_wait();
     if (tid == 0) {
         // Each picture hands out its CTUs by ticket in wavefront order.  CTAs start at picture
         // blockIdx.x % n, so the pictures of a launch progress side by side; a picture whose
@@ -573,9 +583,6 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS + (WARPS > 8)) k_intra_
         cuda::atomic_ref<uint32_t, cuda::thread_scope_device> status(*sticky);
         S.abort = status.load(cuda::memory_order_relaxed) != 0;
     }
-#pragma unroll 1
-    for (int q = tid; q < (int)sizeof(S.taps) / 16; q += THREADS)
-        cp_async16(reinterpret_cast<uint4*>(S.taps) + q, reinterpret_cast<const uint4*>(c_intra_taps.t) + q);
     __syncthreads();
     if (S.ticket < 0 || S.abort) {
         cp_async_wait_all();

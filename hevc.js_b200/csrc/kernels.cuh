@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(128) k_residual(const __grid_constant__ SegTab
     __shared__ __align__(16) int16_t s_coef[TUS][N * N];
     __shared__ int16_t s_tmp[TUS][N * TP];
 
+    pdl_next();
     const int slot = threadIdx.x / N;
     const int j = threadIdx.x % N;
     const Seg& sg = st.s[find_seg(st, blockIdx.x)];
@@ -188,11 +189,10 @@ __global__ void __launch_bounds__(128) k_residual(const __grid_constant__ SegTab
         for (int k = 0; k < N; k++) s_tmp[slot][k * TP + j] = (int16_t)clip3(-32768, 32767, (d[k] + 64) >> 7);
     }
     __syncthreads();
-    if (!live) return;
-
     // second pass: row j, shift 12 (20 - BitDepth), int16 clip
     int r[N];
-    if (bypass) {
+    if (!live) {
+    } else if (bypass) {
 #pragma unroll
         for (int k = 0; k < N; k++) r[k] = s_coef[slot][j * N + k];
     } else if (tskip) {
@@ -207,6 +207,8 @@ __global__ void __launch_bounds__(128) k_residual(const __grid_constant__ SegTab
         for (int k = 0; k < N; k++) r[k] = clip3(-32768, 32767, (d[k] + 2048) >> 12);
     }
 
+    pdl_wait();   // the transforms need only the records; the predictions come from the kernels before
+    if (!live) return;
     if (intra_item) {
         // residual of an intra TU: the wavefront adds it to its prediction.  A row goes out in
         // 16-byte words (8-byte ones for 4x4): residuals lie at multiples of 16 samples
@@ -267,6 +269,8 @@ __global__ void __launch_bounds__(128) k_residual(const __grid_constant__ SegTab
 // Motion grid: one warp per PU writes its 4x4 entries (used by the Bs derivation).
 // ======================================================================================
 __global__ void k_motion_grid(const __grid_constant__ SegTable st) {
+    pdl_next();
+    pdl_wait();
     const PicDesc& P = *st.s[blockIdx.y].pic;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x % 32;
     if (warp >= P.num_pus) return;
@@ -414,6 +418,8 @@ __device__ __forceinline__ void luma_segment(int (&p)[4][4], int (&q)[4][4], int
 #endif
 template <bool VERT>
 __global__ void __launch_bounds__(256, HEVCGPU_DEBLOCK_MIN_CTAS) k_deblock(const __grid_constant__ SegTable st) {
+    pdl_next();
+    pdl_wait();
     const PicDesc& P = *st.s[blockIdx.y].pic;
     const int W = P.width, H = P.height, gw = W >> 2;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -643,6 +649,8 @@ __device__ __forceinline__ uint32_t lanes_join(uint32_t even, uint32_t odd) { re
 // transquant bypass — get their deblocked value back.  Reads the deblocked buffer (rec),
 // writes the DPB slot (dst), so no full-picture copy is made.
 __global__ void __launch_bounds__(256) k_sao(const __grid_constant__ SegTable st) {
+    pdl_next();
+    pdl_wait();
     const PicDesc& P = *st.s[blockIdx.y].pic;
     const int ctb = blockIdx.x;
     if (ctb >= P.wctb * P.hctb) return;

@@ -249,13 +249,11 @@ __device__ __forceinline__ void mc_list(const uint8_t* plane, int pitch, int pw,
     }
 }
 
-// Luma strips and chroma strips are separate launches (separate item lists).
+// The strip of one thread.
 template <bool CHROMA>
-__global__ void __launch_bounds__(MC_THREADS, HEVCGPU_MC_MIN_CTAS) k_mc(const __grid_constant__ SegTable st) {
+__device__ __forceinline__ void mc_strip(const SegTable& st, uint2 (&s_pred)[MC_STRIP_ROWS][MC_THREADS], int tid) {
     using G_ = McGeom<CHROMA>;
     constexpr int SUB = G_::SUB;
-    __shared__ uint2 s_pred[MC_STRIP_ROWS][MC_THREADS];   // list-0 predictions of bi strips
-    const int tid = threadIdx.x;
     const Seg& sg = st.s[find_seg(st, blockIdx.x)];
     const int item = (blockIdx.x - sg.block0) * MC_THREADS + tid;
     if (item >= sg.n_items) return;
@@ -335,6 +333,16 @@ __global__ void __launch_bounds__(MC_THREADS, HEVCGPU_MC_MIN_CTAS) k_mc(const __
         else
             mc_list<CHROMA, false>(ref, pitch, pw, ph, x0, y0, fx, fy, rows, emit);
     }
+}
+
+// Luma strips and chroma strips are separate launches (separate item lists).
+template <bool CHROMA>
+__global__ void __launch_bounds__(MC_THREADS, HEVCGPU_MC_MIN_CTAS) k_mc(const __grid_constant__ SegTable st) {
+    __shared__ uint2 s_pred[MC_STRIP_ROWS][MC_THREADS];   // list-0 predictions of bi strips
+    const int tid = threadIdx.x;
+    pdl_next();
+    mc_strip<CHROMA>(st, s_pred, tid);
+    pdl_wait();   // nothing here needs the kernel before (the plan, or luma): wait last
 }
 
 }  // namespace hevcgpu
