@@ -74,7 +74,7 @@ struct PicDesc {
     int32_t pitch_y, pitch_c;
     int64_t off_cb, off_cr;
     uint8_t* rec;                        // reconstruction / deblocking buffer
-    uint8_t* dst;                        // DPB slot written by SAO
+    uint8_t* dst;                        // packed output of independent blocks (RES_PACKED)
     const uint8_t* ref[2][16];           // reference pictures by list entry (Y base)
     int32_t num_ref[2];
     int32_t ref_poc[2][16];
@@ -137,7 +137,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 
 // A launch covers up to MAX_SEGS pictures.  Segment k owns the blocks
 // [block0, next block0) of an item-list launch, or blockIdx.y == k of a per-picture
-// launch.  The table is a kernel parameter, so a batched launch needs no device-side
+// launch (whose items field is the picture SAO writes).  The table is a kernel parameter, so a batched launch needs no device-side
 // bookkeeping and is captured by value in a CUDA graph.
 constexpr int MAX_SEGS = 64;
 struct Seg {

@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(256) k_sao(const __grid_constant__ SegTable st
     const int pitch = ci ? P.pitch_c : P.pitch_y;
     const int64_t base = ci == 0 ? 0 : (ci == 1 ? P.off_cb : P.off_cr);
     const uint8_t* S = P.rec + base;
-    uint8_t* D = P.dst + base;
+    uint8_t* D = static_cast<uint8_t*>(const_cast<void*>(st.s[blockIdx.y].items)) + base;   // the DPB slot
     if (x >= pw) return;
     const int n = min(8, pw - x);          // 8, or 4 at the end of a row
     const int ymax = min(cy + cs, ph);
