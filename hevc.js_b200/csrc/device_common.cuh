@@ -132,13 +132,28 @@ struct PicDesc {
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// 16-byte asynchronous global -> shared copy (through L2 only, so that samples other
+// CTUs wrote are seen), and the wait for all of a thread's copies.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
+                 "l"(gmem));
+}
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
 // Work items ----------------------------------------------------------------------------
-// Residual items are TU indices (int32), or RES_INTRA_ITEM | task index for intra TUs; motion-compensation items are packed strips (mc_item, mc.cuh).
+// Residual items are TU indices (int32), or RES_INTRA_ITEM | task index for intra TUs;
+// motion-compensation items are packed strips (mc_item, mc.cuh).
 
 // A launch covers up to MAX_SEGS pictures.  Segment k owns the blocks
 // [block0, next block0) of an item-list launch, or blockIdx.y == k of a per-picture
-// launch (whose items field is the picture SAO writes).  The table is a kernel parameter, so a batched launch needs no device-side
-// bookkeeping and is captured by value in a CUDA graph.
+// launch (whose items field is the picture the loop filter writes).  The table is a kernel
+// parameter, so a batched launch needs no device-side bookkeeping and is captured by value in a
+// CUDA graph.
 constexpr int MAX_SEGS = 64;
 struct Seg {
     const void* items;

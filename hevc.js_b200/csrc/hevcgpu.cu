@@ -24,6 +24,7 @@
 #include "intra.cuh"
 #include "mc.cuh"
 #include "kernels.cuh"
+#include "filters.cuh"
 
 using namespace hevcgpu;
 
@@ -1367,25 +1368,37 @@ struct Launcher {
         return HEVCGPU_OK;
     }
 
-    // per-picture launch: grid.y = picture; grid.x from blocks_of(job)
-    template <typename K, typename F>
-    int pictures(K kernel, hevcgpu_job* const* jobs, int n, int threads, int z, F blocks_of) {
+    // per-picture launch: grid.y = picture, grid.x from blocks_of(job); launch(grid, table,
+    // blocks at work)
+    template <typename F, typename G>
+    int pictures(hevcgpu_job* const* jobs, int n, F blocks_of, G launch) {
         for (int b0 = 0; b0 < n; b0 += MAX_SEGS) {
             SegTable t;
             std::memset(&t, 0, sizeof(t));
-            int bx = 0;
+            int bx = 0, sum = 0;
             for (int k = b0; k < std::min(n, b0 + MAX_SEGS); k++) {
                 Seg& sg = t.s[t.n++];
                 sg.pic = jobs[k]->d_desc;
                 sg.items = jobs[k]->dst;
-                bx = std::max(bx, blocks_of(jobs[k]));
+                const int blocks = blocks_of(jobs[k]);
+                bx = std::max(bx, blocks);
+                sum += blocks;
             }
-            int rc = go(kernel, dim3(bx, t.n, z), dim3(threads), t);
+            int rc = launch(dim3(bx, t.n), t, sum);
             if (rc) return rc;
         }
         return HEVCGPU_OK;
     }
 };
+
+// Dynamic shared memory of a loop filter launch: as much as leaves room for just the per_sm CTAs
+// an SM has to take.  The launch may start while the intra stage still holds most SMs, and would
+// otherwise put all of a small launch's CTAs on the few that are free: 4 streams' GOPs at 720p
+// (960 tiles a launch) 1,160 us without it, 1,125 with it.
+size_t lf_pad(int per_sm, int threads) {
+    if (per_sm >= lf_ctas(threads)) return 0;
+    return (228 * 1024 / per_sm - 1024 - sizeof(LfSmem)) & ~(size_t)127;
+}
 
 // Brackets one stage with profiling events when profiling is on.
 struct StageMark {
@@ -1485,7 +1498,9 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
     }
     if ((stages & ST_DEBLOCK) && !(stages & ST_MC)) {   // with MC, its luma strips write the grid
         StageMark m(ctx, ex.stream, 0);
-        rc = L.pictures(k_motion_grid, jobs, n, 256, 1, [](hevcgpu_job* j) { return (j->n_pus * 32 + 255) / 256; });
+        rc = L.pictures(
+            jobs, n, [](hevcgpu_job* j) { return (j->n_pus * 32 + 255) / 256; },
+            [&](dim3 grid, const SegTable& t, int) { return L.go(k_motion_grid, grid, dim3(256), t); });
         if (rc) return rc;
     }
     if (stages & ST_MC) {
@@ -1523,29 +1538,22 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
                                 ex.tickets(), g.total, sticky);
         if (rc) return rc;
     }
-    if (stages & ST_DEBLOCK) {
-        {
-            StageMark m(ctx, ex.stream, 4);
-            rc = L.pictures(k_deblock<true>, jobs, n, 256, 1, [](hevcgpu_job* j) {
-                int segs = ((j->params.width + 7) / 8) * (j->params.height / 4);
-                return (segs + 255) / 256;
+    if (stages & ST_SAO) {   // deblocking, when asked for, then SAO into the slot
+        StageMark m(ctx, ex.stream, stages & ST_DEBLOCK ? 4 : 6);
+        rc = L.pictures(
+            jobs, n,
+            [](hevcgpu_job* j) {
+                return ((j->params.width + LF_T - 1) / LF_T) * ((j->params.height + LF_T - 1) / LF_T);
+            },
+            [&](dim3 grid, const SegTable& t, int tiles) {
+                const int per_sm = (tiles + ctx->sm_count - 1) / ctx->sm_count, deblock = stages & ST_DEBLOCK ? 1 : 0;
+                auto go = [&](auto* kernel, int threads) {
+                    return L.go_smem(kernel, grid, dim3(threads), lf_pad(per_sm, threads), t, deblock);
+                };
+                // 256 threads while all tiles are resident at once, else 128 (lf_ctas)
+                if (per_sm <= lf_ctas(256)) return go(k_loop_filter<256>, 256);
+                return go(k_loop_filter<128>, 128);
             });
-            if (rc) return rc;
-        }
-        StageMark m(ctx, ex.stream, 5);
-        rc = L.pictures(k_deblock<false>, jobs, n, 256, 1, [](hevcgpu_job* j) {
-            int segs = (j->params.width / 4) * ((j->params.height + 7) / 8);
-            return (segs + 255) / 256;
-        });
-        if (rc) return rc;
-    }
-    if (stages & ST_SAO) {
-        StageMark m(ctx, ex.stream, 6);
-        // one CTA per CTB; z = 0 luma, z = 1 both chroma planes
-        rc = L.pictures(k_sao, jobs, n, 256, 2, [](hevcgpu_job* j) {
-            const int ctb = 1 << j->params.log2_ctb;
-            return ((j->params.width + ctb - 1) / ctb) * ((j->params.height + ctb - 1) / ctb);
-        });
         if (rc) return rc;
     }
     return HEVCGPU_OK;
@@ -1623,6 +1631,8 @@ int hevcgpu_create(int device, hevcgpu_ctx_t** out) {
                                   (int)sizeof(IntraSmem)));
     CUDA_TRY(cudaFuncSetAttribute(k_intra_ctus<IC_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sizeof(IntraSmem)));
+    for (auto* k : {k_loop_filter<128>, k_loop_filter<256>})
+        CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lf_pad(1, 128)));
     auto* c = new (std::nothrow) hevcgpu_ctx();
     if (!c) return fail(HEVCGPU_ENOMEM, "host allocation");
     c->device = device;

@@ -260,19 +260,6 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// 16-byte asynchronous global -> shared copy (through L2 only, so that samples other
-// CTUs wrote are seen), and the wait for all of a thread's copies.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
-                 "l"(gmem));
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
 // Barriers in shared memory, one per TU of the CTU that waits for others, with as many
 // arrivals as the TUs it waits for: each arrives when it completes (release), the TU's warp
 // waits on phase 0 (acquire).  A waiting thread is suspended by the hardware until the phase

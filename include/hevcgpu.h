@@ -423,8 +423,8 @@ uint64_t hevcgpu_launch_count(hevcgpu_ctx_t* ctx);
  * each reconstruction stage of every later launch.  hevcgpu_profile_read waits for the
  * stream and returns, per stage, the summed device milliseconds and the number of kernel
  * launches since the previous read.  Stages: 0 motion grid, 1 motion compensation,
- * 2 residual, 3 intra wavefront, 4 deblocking (vertical edges), 5 deblocking
- * (horizontal edges), 6 SAO. */
+ * 2 residual, 3 intra wavefront, 4 loop filter (deblocking and SAO, one kernel), 5 always
+ * 0, 6 SAO of a launch without deblocking. */
 #define HEVCGPU_NUM_STAGES 7
 int hevcgpu_profile_enable(hevcgpu_ctx_t* ctx, int enable);
 int hevcgpu_profile_read(hevcgpu_ctx_t* ctx, double* ms, uint64_t* launches);
