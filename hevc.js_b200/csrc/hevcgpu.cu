@@ -793,13 +793,18 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
         uint32_t* own = owner[c].data();
         const int row = uw[c];
         int dp = 0;
-        uint32_t last = 0, last_seg = 0;   // a run of units with one owner adds what its first unit added
+        uint32_t last = 0;   // a run of units with one owner adds what its first unit added
+        int32_t spare = 0, *last_at = &spare;
         // seg: the part of b's reference array the unit lies in (SEG_*); an owner's entry carries
         // all parts it owns samples of
         auto dep = [&](uint32_t o, uint32_t seg) {
-            if ((o & GEN_BITS) != gtag || (o == last && seg == last_seg)) return;
+            if ((o & GEN_BITS) != gtag) return;
+            if (o == last) {
+                *last_at |= (int32_t)(seg << INTRA_DEP_SEG_SHIFT);
+                return;
+            }
             last = o;
-            last_seg = seg;
+            last_at = &spare;
             const int32_t ob = (int32_t)(o & 0xFFFFFFu);
             const int oa = ctu_of[(size_t)ob];
             // a CTU later in raster order is never available to this one
@@ -810,22 +815,24 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
             for (size_t q = first_dep; q < n_own; q++)
                 if ((D[q] & OWNER) == ob) {
                     D[q] |= (int32_t)(seg << INTRA_DEP_SEG_SHIFT);
+                    last_at = &D[q];
                     return;
                 }
+            last_at = &D[n_own];
             D[n_own++] = ob | (int32_t)(seg << INTRA_DEP_SEG_SHIFT);
             dp = std::max(dp, level[(size_t)ob] + 1);   // local and external dependencies alike
         };
-        const int ux = t.x / 4, uy = t.y / 4;
-        if (t.y > 0) {
-            const size_t rrow = (size_t)((t.y - 1) / 4) * row;
-            const int ux0 = t.x > 0 ? (t.x - 1) / 4 : 0, ux1 = std::min(row - 1, (t.x + 2 * n - 1) / 4);
-            const int uxn = ux + n / 4;   // the corner is the unit left of ux
-            for (int x = ux0; x <= ux1; x++) dep(own[rrow + x], x < ux ? SEG_C : (x < uxn ? SEG_T : SEG_TR));
+        const int ux = t.x / 4, uy = t.y / 4, nu = n / 4;
+        if (uy > 0) {
+            const uint32_t* r = own + (size_t)(uy - 1) * row;
+            if (ux > 0) dep(r[ux - 1], SEG_C);
+            for (int x = ux; x < ux + nu; x++) dep(r[x], SEG_T);
+            for (int x = ux + nu; x < std::min(row, ux + 2 * nu); x++) dep(r[x], SEG_TR);
         }
-        if (t.x > 0) {
-            const int lx = (t.x - 1) / 4, uy0 = t.y / 4, uy1 = std::min(uh[c] - 1, (t.y + 2 * n - 1) / 4);
-            const int uyn = uy + n / 4;
-            for (int y = uy0; y <= uy1; y++) dep(own[(size_t)y * row + lx], y < uyn ? SEG_L : SEG_BL);
+        if (ux > 0) {
+            const uint32_t* r = own + (size_t)uy * row + ux - 1;
+            for (int y = 0; y < nu; y++, r += row) dep(*r, SEG_L);
+            for (int y = uy + nu; y < std::min(uh[c], uy + 2 * nu); y++, r += row) dep(*r, SEG_BL);
         }
         level[(size_t)b] = dp;
         BS.depth = std::max(BS.depth, dp + 1);
@@ -932,14 +939,17 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
     watch.clear();
     ictu_watch.assign((size_t)nic, 0u);
     slot_of.assign((size_t)n_intra, -1);
+    int n_item = 0;
+    BS.items.resize((size_t)n_intra * intra_bands(5));
+    uint16_t* items = BS.items.data();
     for (int k = 0; k < nic; k++) {
         int acc = 0, nw = 0;
         const uint32_t w0 = (uint32_t)watch.size(), nd0 = nd;
-        const int item0 = (int)BS.items.size();
+        const int item0 = n_item;
         const int t0 = ictu_tu_off[(size_t)k], t1 = ictu_tu_off[(size_t)k + 1];
         if (t1 - t0 > IC_MAX_TUS)
             return fail(HEVCGPU_EINVAL, "CTU %d holds more intra TUs than a CTU can", ictu_addr[(size_t)k]);
-        const int a = ictu_addr[(size_t)k];
+        const int a = ictu_addr[(size_t)k], ax = a % wctb, ay = a / wctb;
         for (int i = t0; i < t1; i++) {
             const int b = order[(size_t)i];
             const hevc_tu_t& t = s->tus[itu[(size_t)i]];
@@ -949,10 +959,12 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
             r.reserved[0] = 0;
             const int d0 = dep_at[(size_t)b], d1 = dep_at[(size_t)b + 1];
             itu_dep[(size_t)i] = (nd << 6) | (uint32_t)(d1 - d0);
+            const uint32_t task = (uint32_t)(i - t0) << INTRA_DEP_TASK_SHIFT;
             for (int q = d0; q < d1; q++) {
-                const int ob = deps[(size_t)q] & OWNER, oi = pos[(size_t)ob];
-                const uint32_t segs = (uint32_t)(deps[(size_t)q] & ~OWNER) | (uint32_t)(i - t0) << INTRA_DEP_TASK_SHIFT;
-                if (ctu_of[(size_t)ob] == a) {
+                const int32_t e = D[q];
+                const int oi = pos[(size_t)(e & OWNER)];
+                const uint32_t segs = (uint32_t)(e & ~OWNER) | task;
+                if (oi >= t0) {   // a TU of this CTU
                     dout[nd++] = segs | (uint32_t)(oi - t0);
                     continue;
                 }
@@ -964,15 +976,16 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
                     so = (k << 8) | nw++;
                     watch.push_back((uint32_t)oi);
                     const hevc_tu_t& o = itu_rec[(size_t)oi];
-                    const int cs = ctb >> (o.c_idx ? 1 : 0);
-                    BS.watch_geo.push_back(intra_watch_pack({o.c_idx, (1 << o.log2_size) / 4, (o.x - a % wctb * cs) / 4,
-                                                             (o.y - a / wctb * cs) / 4}));
+                    const int lu = p.log2_ctb - (o.c_idx ? 1 : 0) - 2;   // CTB in 4-sample units
+                    BS.watch_geo.push_back(intra_watch_pack({o.c_idx, (1 << o.log2_size) / 4, o.x / 4 - (ax << lu),
+                                                             o.y / 4 - (ay << lu)}));
                     itu_rec[(size_t)oi].reserved[0] = ITU_PUBLISH;
                 }
                 dout[nd++] = segs | (uint32_t)(IC_MAX_TUS + (so & 0xFF));
             }
-            for (int band = 0; band < intra_bands(t.log2_size); band++)
-                BS.items.push_back((uint16_t)((i - t0) | band << INTRA_DEP_TASK_SHIFT));
+            items[n_item++] = (uint16_t)(i - t0);
+            for (int band = 1; band < intra_bands(t.log2_size); band++)
+                items[n_item++] = (uint16_t)((i - t0) | band << INTRA_DEP_TASK_SHIFT);
             if (!(t.flags & HEVC_TU_CODED)) continue;
             const int nn = 1 << (2 * t.log2_size);
             itu_res[(size_t)i] = make_int2((int)t.coeff_offset, res_total + acc);
@@ -983,9 +996,10 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
             return fail(HEVCGPU_EINVAL, "CTU %d holds more intra TUs than a CTU can", a);
         ictu_watch[(size_t)k] = (w0 << 8) | (uint32_t)nw;
         BS.ictu.push_back({a, t0, t1 - t0, (int32_t)(nd - nd0), nd0, w0, nw, neighbours(a), res_total, acc, item0,
-                           (int32_t)BS.items.size() - item0});
+                           n_item - item0});
         res_total += acc;
     }
+    BS.items.resize((size_t)n_item);
     BS.res_total = res_total;
     // one spare entry: an external dependency of task 0 on itself (the planted wait of
     // hevcgpu_job_plant_unmet_wait points task 0's list at it)
