@@ -419,7 +419,7 @@ struct hevcgpu_job {
     cudaEvent_t direct_read = nullptr;  // the uploads straight from the caller's arrays are done
     PicDesc host_desc{};
     int32_t n_res[4] = {0, 0, 0, 0};
-    const int32_t* d_res[4] = {nullptr, nullptr, nullptr, nullptr};
+    const int32_t* d_res = nullptr;   // 32x32 first, then 16x16, 8x8, 4x4
     int32_t n_mc[2] = {0, 0};            // luma strips, chroma strips (mc.cuh items)
     const uint32_t* d_mc[2] = {nullptr, nullptr};
     int32_t n_ictu = 0;                 // CTUs that hold intra TUs
@@ -464,6 +464,16 @@ struct Packer {
         size_t off = (size_t)align_up((int64_t)size, 256);
         size = off + bytes;
         if (out && bytes && src) std::memcpy(out + off, src, bytes);
+        return off;
+    }
+    // lists by size, largest first, back to back
+    size_t add_joined(const std::vector<int32_t> (&lists)[4]) {
+        const size_t off = add(nullptr, 0);
+        for (int k = 3; k >= 0; k--) {
+            const size_t bytes = sizeof(int32_t) * lists[k].size();
+            if (out && bytes) std::memcpy(out + size, lists[k].data(), bytes);
+            size += bytes;
+        }
         return off;
     }
 };
@@ -1159,7 +1169,7 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     }
     j->n_pus = s->num_pus;
 
-    size_t o_wp, o_sao, o_sl, o_ti, o_slices, o_res[4], o_mc[2], o_ia, o_idp, o_itu, o_iro, o_dl, o_wl, o_it;
+    size_t o_wp, o_sao, o_sl, o_ti, o_slices, o_res, o_mc[2], o_ia, o_idp, o_itu, o_iro, o_dl, o_wl, o_it;
     size_t o_scal = 0;
     hevc_slice_t dflt{0, 0, 0, 1};
     const bool scaled = s->scaling && (stages & (ST_RESID | ST_INTRA));
@@ -1171,7 +1181,7 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
         o_ti = pk.add(s->ctb_tile, s->ctb_tile ? sizeof(uint16_t) * (size_t)nctb : 0);
         o_slices = s->num_slices > 0 && s->slices ? pk.add(s->slices, sizeof(hevc_slice_t) * (size_t)s->num_slices)
                                                   : pk.add(&dflt, sizeof(dflt));
-        for (int k = 0; k < 4; k++) o_res[k] = pk.add(bins[k].data(), sizeof(int32_t) * bins[k].size());
+        o_res = pk.add_joined(bins);
         for (int c = 0; c < 2; c++) o_mc[c] = pk.add(mc[c].data(), sizeof(uint32_t) * mc[c].size());
         o_ia = pk.add(ictu.data(), sizeof(IntraCtu) * ictu.size());
         o_itu = pk.add(itu_rec.data(), sizeof(hevc_tu_t) * itu_rec.size());
@@ -1275,10 +1285,8 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
         }
     }
     D.pcm_bypass_any = pcm_bypass ? 1 : 0;
-    for (int k = 0; k < 4; k++) {
-        j->n_res[k] = (int32_t)bins[k].size();
-        j->d_res[k] = reinterpret_cast<const int32_t*>(base + o_res[k]);
-    }
+    for (int k = 0; k < 4; k++) j->n_res[k] = (int32_t)bins[k].size();
+    j->d_res = reinterpret_cast<const int32_t*>(base + o_res);
     for (int c = 0; c < 2; c++) {
         j->n_mc[c] = (int32_t)mc[c].size();
         j->d_mc[c] = reinterpret_cast<const uint32_t*>(base + o_mc[c]);
@@ -1414,6 +1422,21 @@ size_t lf_pad(int per_sm, int threads) {
     return (228 * 1024 / per_sm - 1024 - sizeof(LfSmem)) & ~(size_t)127;
 }
 
+// Adds a picture's coded TUs (items: by size, largest first) to a residual launch of `blocks`
+// CTAs so far; returns the new number.
+int res_add(ResTable& t, int blocks, const int32_t* items, const PicDesc* pic, const int32_t (&n)[4]) {
+    if (n[0] + n[1] + n[2] + n[3] == 0) return blocks;
+    ResSeg& sg = t.s[t.n++];
+    sg.items = reinterpret_cast<const uint32_t*>(items);
+    sg.pic = pic;
+    sg.block0 = blocks;
+    for (int k = 0; k < 4; k++) {
+        sg.n[k] = n[k];
+        blocks += res_blocks(n[k], k + 2);
+    }
+    return blocks;
+}
+
 // Brackets one stage with profiling events when profiling is on.
 struct StageMark {
     hevcgpu_ctx* ctx;
@@ -1532,15 +1555,13 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
     }
     if (stages & (ST_RESID | ST_INTRA)) {
         StageMark m(ctx, ex.stream, 2);
-        void (*kr[4])(const SegTable, int) = {k_residual<2>, k_residual<3>, k_residual<4>, k_residual<5>};
-        for (int k = 0; k < 4; k++) {
-            rc = L.items(kr[k], jobs, n, 128 >> (k + 2), 128,
-                         [k](hevcgpu_job* j, const void*& p, int& c) {
-                             p = j->d_res[k];
-                             c = j->n_res[k];
-                         },
-                         res_mode);
-            if (rc) return rc;
+        for (int b0 = 0; b0 < n; b0 += MAX_SEGS) {
+            ResTable t;
+            std::memset(&t, 0, sizeof(t));
+            int blocks = 0;
+            for (int k = b0; k < std::min(n, b0 + MAX_SEGS); k++)
+                blocks = res_add(t, blocks, jobs[k]->d_res, jobs[k]->d_desc, jobs[k]->n_res);
+            if ((rc = L.go(k_residual, dim3(blocks), dim3(RES_THREADS), t, res_mode))) return rc;
         }
     }
     for (const IntraLaunch& g : intra) {
@@ -1715,14 +1736,14 @@ int hevcgpu_residual_blocks_scaled(hevcgpu_ctx_t* ctx, const hevc_scaling_t* sca
     j.ctx = ctx;
     std::vector<int32_t> bins[4];
     for (int i = 0; i < num_tus; i++) bins[tus[i].log2_size - 2].push_back(i);
-    size_t o_tus, o_coef, o_pred, o_out, o_res[4], o_scal = 0;
+    size_t o_tus, o_coef, o_pred, o_out, o_res, o_scal = 0;
     auto pack = [&](Packer& pk) {
         if (scaling) o_scal = pk.add(scaling, sizeof(hevc_scaling_t));
         o_tus = pk.add(tus, sizeof(hevc_tu_t) * (size_t)num_tus);
         o_coef = pk.add(coeffs, sizeof(int16_t) * (size_t)num_coeffs);
         o_pred = pk.add(pred, (size_t)num_coeffs);
         o_out = pk.add(nullptr, (size_t)num_coeffs);
-        for (int k = 0; k < 4; k++) o_res[k] = pk.add(bins[k].data(), sizeof(int32_t) * bins[k].size());
+        o_res = pk.add_joined(bins);
     };
     Packer measure;
     pack(measure);
@@ -1742,10 +1763,8 @@ int hevcgpu_residual_blocks_scaled(hevcgpu_ctx_t* ctx, const hevc_scaling_t* sca
     D.rec = base + o_pred;
     D.dst = base + o_out;
     D.scaling = scaling ? reinterpret_cast<const hevc_scaling_t*>(base + o_scal) : nullptr;
-    for (int k = 0; k < 4; k++) {
-        j.n_res[k] = (int32_t)bins[k].size();
-        j.d_res[k] = reinterpret_cast<const int32_t*>(base + o_res[k]);
-    }
+    for (int k = 0; k < 4; k++) j.n_res[k] = (int32_t)bins[k].size();
+    j.d_res = reinterpret_cast<const int32_t*>(base + o_res);
     CUDA_TRY(cudaMemcpyAsync(j.recs.p, j.pin.p, img, cudaMemcpyHostToDevice, ctx->stream));
     std::memcpy(static_cast<uint8_t*>(j.pin.p) + j.desc_off, &D, sizeof(D));
     CUDA_TRY(cudaMemcpyAsync(j.desc.p, static_cast<uint8_t*>(j.pin.p) + j.desc_off, sizeof(D),
@@ -1855,12 +1874,11 @@ int hevcgpu_residual_blocks_static(hevcgpu_ctx_t* ctx, const hevc_tu_t* tus, int
     }
     const SyncOnExit drained{ctx->stream};   // declared after the lock: runs before it is released
 
-    // per-size lists of TU indices, back to back in the device's list array
-    int32_t count[4] = {0, 0, 0, 0}, start[4];
+    // per-size lists of TU indices, largest first, back to back in the device's list array
+    int32_t count[4] = {0, 0, 0, 0}, fill[4];
     for (int i = 0; i < num_tus; i++) count[tus[i].log2_size - 2]++;
-    start[0] = 0;
-    for (int k = 1; k < 4; k++) start[k] = start[k - 1] + count[k - 1];
-    int32_t fill[4] = {start[0], start[1], start[2], start[3]};
+    fill[3] = 0;
+    for (int k = 2; k >= 0; k--) fill[k] = fill[k + 1] + count[k + 1];
     for (int i = 0; i < num_tus; i++) sd.lists[fill[tus[i].log2_size - 2]++] = i;
 
     PicDesc D;
@@ -1877,20 +1895,11 @@ int hevcgpu_residual_blocks_static(hevcgpu_ctx_t* ctx, const hevc_tu_t* tus, int
                              cudaMemcpyHostToDevice, ctx->stream));
 
     Launcher L{ctx, ctx->stream};
-    void (*kr[4])(const SegTable, int) = {k_residual<2>, k_residual<3>, k_residual<4>, k_residual<5>};
-    for (int k = 0; k < 4; k++) {
-        if (count[k] == 0) continue;
-        const int per_block = 128 >> (k + 2);
-        SegTable t;
-        std::memset(&t, 0, sizeof(t));
-        t.n = 1;
-        t.s[0].items = base + STATIC_LISTS_OFF + sizeof(int32_t) * (size_t)start[k];
-        t.s[0].pic = reinterpret_cast<const PicDesc*>(base);
-        t.s[0].n_items = count[k];
-        t.s[0].block0 = 0;
-        if ((rc = L.go(kr[k], dim3((count[k] + per_block - 1) / per_block), dim3(128), t, (int)RES_PACKED)))
-            return rc;
-    }
+    ResTable t;
+    std::memset(&t, 0, sizeof(t));
+    const int blocks = res_add(t, 0, reinterpret_cast<const int32_t*>(base + STATIC_LISTS_OFF),
+                               reinterpret_cast<const PicDesc*>(base), count);
+    if ((rc = L.go(k_residual, dim3(blocks), dim3(RES_THREADS), t, (int)RES_PACKED))) return rc;
     // the lock is held until the kernels are done with the scratch (and `drained` waits
     // again on the way out of every earlier return)
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
