@@ -1437,6 +1437,18 @@ int res_add(ResTable& t, int blocks, const int32_t* items, const PicDesc* pic, c
     return blocks;
 }
 
+// Parts (a power of two) that the strips of an MC launch are divided into, each a thread's.  A
+// part reads NT - 1 rows more than it writes, so parts cost work; but a thread takes some 9 us for
+// a bi-predicted strip of 16 rows, and few strips leave most of the chip idle meanwhile.  Four
+// parts while all strips fill at most one CTA per SM, two up to four: luma and chroma of one
+// 416x240 picture 23 us whole, 17 in two parts, 13 in four; one 1280x720 23 / 21 / 19, two
+// 27 / 23 / 23, three 36 / 28 / 33; one 1080p 28 / 24 / 25, two 37 / 38 / 37; one 2160p (6 CTAs
+// per SM) 46 / 46 / 56.
+int mc_split(int64_t strips, int sms) {
+    const int64_t ctas = (strips + MC_THREADS - 1) / MC_THREADS;
+    return ctas <= sms ? 2 : (ctas <= 4 * sms ? 1 : 0);
+}
+
 // Brackets one stage with profiling events when profiling is on.
 struct StageMark {
     hevcgpu_ctx* ctx;
@@ -1542,16 +1554,20 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
     }
     if (stages & ST_MC) {
         StageMark m(ctx, ex.stream, 1);
-        rc = L.items(k_mc<false>, jobs, n, MC_THREADS, MC_THREADS, [](hevcgpu_job* j, const void*& p, int& c) {
-            p = j->d_mc[0];
-            c = j->n_mc[0];
-        });
-        if (rc) return rc;
-        rc = L.items(k_mc<true>, jobs, n, MC_THREADS, MC_THREADS, [](hevcgpu_job* j, const void*& p, int& c) {
-            p = j->d_mc[1];
-            c = j->n_mc[1];
-        });
-        if (rc) return rc;
+        for (int c = 0; c < 2; c++) {
+            int64_t strips = 0;
+            for (int k = 0; k < n; k++) strips += jobs[k]->n_mc[c];
+            const int split = mc_split(strips, ctx->sm_count);
+            auto* const kernel = c ? (split ? k_mc<true, true> : k_mc<true, false>)
+                                   : (split ? k_mc<false, true> : k_mc<false, false>);
+            rc = L.items(kernel, jobs, n, MC_THREADS >> split, MC_THREADS,
+                         [c](hevcgpu_job* j, const void*& p, int& cnt) {
+                             p = j->d_mc[c];
+                             cnt = j->n_mc[c];
+                         },
+                         split);
+            if (rc) return rc;
+        }
     }
     if (stages & (ST_RESID | ST_INTRA)) {
         StageMark m(ctx, ex.stream, 2);

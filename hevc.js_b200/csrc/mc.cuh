@@ -2,7 +2,8 @@
 // src/decoding/interpolation.cpp:306-411; interpolate_luma :45-127, interpolate_chroma
 // :133-209, weighted_pred_default :215-240, weighted_pred_explicit :246-300).
 //
-// One thread per strip: 4 columns x up to 16 rows of one PU in one plane.  Per reference
+// One thread per strip: 4 columns x up to 16 rows of one PU in one plane (of a launch with few
+// strips, per half or quarter of one: mc_split).  Per reference
 // list the thread walks the rows of its reference window once, two rows at a time:
 //   1. the two rows are read as aligned 32-bit words (the next two rows' loads are issued
 //      before these are used, so a row's latency overlaps the previous rows' arithmetic);
@@ -249,19 +250,24 @@ __device__ __forceinline__ void mc_list(const uint8_t* plane, int pitch, int pw,
     }
 }
 
-// The strip of one thread.
+// The strip of one thread, or with split > 0 the part of it: the strips of a CTA's first
+// MC_THREADS >> split threads, whose later parts its other warps do.
 template <bool CHROMA>
-__device__ __forceinline__ void mc_strip(const SegTable& st, uint2 (&s_pred)[MC_STRIP_ROWS][MC_THREADS], int tid) {
+__device__ __forceinline__ void mc_strip(const SegTable& st, uint2 (&s_pred)[MC_STRIP_ROWS][MC_THREADS], int tid,
+                                         int split) {
     using G_ = McGeom<CHROMA>;
     constexpr int SUB = G_::SUB;
     const Seg& sg = st.s[find_seg(st, blockIdx.x)];
-    const int item = (blockIdx.x - sg.block0) * MC_THREADS + tid;
+    const int per_cta = MC_THREADS >> split, part = tid / per_cta;
+    const int item = (blockIdx.x - sg.block0) * per_cta + (tid & (per_cta - 1));
     if (item >= sg.n_items) return;
     const uint32_t it = static_cast<const uint32_t*>(sg.items)[item];
     const PicDesc& P = *sg.pic;
     const hevc_pu_t pu = P.pus[it & (MC_MAX_PUS - 1)];
-    const int sx = (int)((it >> 20) & 15) << 2, sy = (int)((it >> 24) & 3) << 4;
-    const int rows = CHROMA ? 2 * (int)(((it >> 26) & 7) + 1) : 4 * (int)(((it >> 26) & 7) + 1);
+    const int above = part * (MC_STRIP_ROWS >> split);   // rows of the strip above the part
+    const int sx = (int)((it >> 20) & 15) << 2, sy = ((int)((it >> 24) & 3) << 4) + above;
+    const int rows = min((CHROMA ? 2 : 4) * (int)(((it >> 26) & 7) + 1) - above, MC_STRIP_ROWS >> split);
+    if (rows <= 0) return;
     const int ci = CHROMA ? 1 + (int)((it >> 29) & 1) : 0;
     const bool use0 = pu.ref_idx[0] >= 0, use1 = pu.ref_idx[1] >= 0, bi = use0 && use1;
     const int pw = P.width / SUB, ph = P.height / SUB, pitch = CHROMA ? P.pitch_c : P.pitch_y;
@@ -336,12 +342,14 @@ __device__ __forceinline__ void mc_strip(const SegTable& st, uint2 (&s_pred)[MC_
 }
 
 // Luma strips and chroma strips are separate launches (separate item lists).
-template <bool CHROMA>
-__global__ void __launch_bounds__(MC_THREADS, HEVCGPU_MC_MIN_CTAS) k_mc(const __grid_constant__ SegTable st) {
+// SPLIT: in 1 << split parts; a kernel of its own, since with `split` in registers the whole form
+// spills more (16 1080p P/B pictures 155 us instead of 151).
+template <bool CHROMA, bool SPLIT>
+__global__ void __launch_bounds__(MC_THREADS, HEVCGPU_MC_MIN_CTAS) k_mc(const __grid_constant__ SegTable st, int split) {
     __shared__ uint2 s_pred[MC_STRIP_ROWS][MC_THREADS];   // list-0 predictions of bi strips
     const int tid = threadIdx.x;
     pdl_next();
-    mc_strip<CHROMA>(st, s_pred, tid);
+    mc_strip<CHROMA>(st, s_pred, tid, SPLIT ? split : 0);
     pdl_wait();   // nothing here needs the kernel before (the plan, or luma): wait last
 }
 
