@@ -379,7 +379,7 @@ constexpr int IP_THREADS = 128;
 __global__ void __launch_bounds__(IP_THREADS) k_intra_plan(const __grid_constant__ SegTable st, int32_t* tickets,
                                                              int later, uint32_t* sticky) {
     __shared__ uint32_t s_av[IC_MAX_TUS], s_count[IC_SOURCES], s_fill[IC_SOURCES], s_total, s_bad;
-    __shared__ uint8_t s_edge[IC_EDGES];
+    __shared__ __align__(4) uint8_t s_edge[IC_EDGES];
     const int tid = threadIdx.x, lane = tid % 32;
     pdl_next();   // MC and the residuals' transforms need nothing of the plan
     if (later) pdl_wait();   // the tickets are in use by the group before
@@ -389,9 +389,10 @@ __global__ void __launch_bounds__(IP_THREADS) k_intra_plan(const __grid_constant
     const int idx = blockIdx.x - st.s[k].block0;
     const IntraCtu C = static_cast<const IntraCtu*>(st.s[k].items)[idx];
     const int n_tu = min(C.n_tu, IC_MAX_TUS), n_watch = min(C.n_watch, IC_MAX_WATCH);
+    auto source = [&](int q) { return q < n_tu ? q : IC_MAX_TUS + q - n_tu; };   // the CTU's TUs, then those it watches
 #pragma unroll 1
-    for (int q = tid; q < IC_SOURCES; q += IP_THREADS) s_count[q] = 0;
-    if (tid < IC_EDGES) s_edge[tid] = 0xFF;
+    for (int q = tid; q < n_tu + n_watch; q += IP_THREADS) s_count[source(q)] = 0;
+    if (tid < IC_EDGES / 4) reinterpret_cast<uint32_t*>(s_edge)[tid] = 0xFFFFFFFFu;
     if (tid == 0) s_total = s_bad = 0;
 #pragma unroll 1
     for (int i = tid; i < n_tu; i += IP_THREADS) {
@@ -434,8 +435,10 @@ __global__ void __launch_bounds__(IP_THREADS) k_intra_plan(const __grid_constant
     // room in rev for each source's waiting TUs (sources in any order: a warp takes its
     // sources' room at once), and the border words the watched TUs stand for
 #pragma unroll 1
-    for (int s = tid; s < IC_SOURCES; s += IP_THREADS) {
-        const uint32_t count = s_count[s];
+    for (int q = tid; q - lane < n_tu + n_watch; q += IP_THREADS) {
+        const bool live = q < n_tu + n_watch;
+        const int s = source(live ? q : 0);
+        const uint32_t count = live ? s_count[s] : 0u;
         uint32_t end = count;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -445,10 +448,11 @@ __global__ void __launch_bounds__(IP_THREADS) k_intra_plan(const __grid_constant
         uint32_t first = 0;
         if (lane == 31 && end) first = atomicAdd(&s_total, end);
         first = __shfl_sync(0xffffffffu, first, 31) + end - count;
+        if (!live) continue;
         s_fill[s] = first;
         s_count[s] = (first << 16) | count;
         const int j = s - IC_MAX_TUS;
-        if (j >= 0 && j < n_watch) {
+        if (j >= 0) {
             const IntraWatch w = intra_watch_unpack(P.watch[C.watch_first + j]);
             const int cw = (1 << (P.log2_ctb - (w.c ? 1 : 0))) / 4;   // words across the CTU
             uint8_t* const edge = s_edge + (w.c == 0 ? 0 : IC_EDGE_L + (w.c - 1) * IC_EDGE_C);
