@@ -70,9 +70,12 @@ __device__ __forceinline__ int dp2a_hi(uint32_t a, uint32_t b, int c) {
 // (24-25), rows code (26-28: luma rows / 4 - 1, chroma rows / 2 - 1), chroma plane (29:
 // 0 Cb, 1 Cr).  Offsets and rows are in samples of the strip's plane.
 constexpr int MC_THREADS = 128;
-#ifndef HEVCGPU_MC_MIN_CTAS
-#define HEVCGPU_MC_MIN_CTAS 6   // CTAs per SM the register budget is sized for (80 registers)
-#endif
+// CTAs per SM that the register budgets are sized for.  Whole luma strips keep a window of 20
+// words and spill with less than the 102 registers of 5; chroma ones need the latency hidden more.
+// 16 1080p P/B pictures, us: 141 with 5 and 8, 144 with 6 and 8, 146 with 4 and 8, 147 with 6 and
+// 9, 152 with 6 and 6.  In parts, beside the kernels before and after, 6: four streams' GOPs at
+// 720p 1,005, 1,048 with 5 for luma, 1,043 with 8 for chroma.
+__host__ __device__ constexpr int mc_ctas(bool chroma, bool split) { return split ? 6 : (chroma ? 8 : 5); }
 constexpr int MC_STRIP_ROWS = 16;
 constexpr int MC_MAX_PUS = 1 << 20;
 __host__ __device__ constexpr uint32_t mc_item(int pu, int sx, int sy, int rows, bool chroma, int plane) {
@@ -345,7 +348,7 @@ __device__ __forceinline__ void mc_strip(const SegTable& st, uint2 (&s_pred)[MC_
 // SPLIT: in 1 << split parts; a kernel of its own, since with `split` in registers the whole form
 // spills more (16 1080p P/B pictures 155 us instead of 151).
 template <bool CHROMA, bool SPLIT>
-__global__ void __launch_bounds__(MC_THREADS, HEVCGPU_MC_MIN_CTAS) k_mc(const __grid_constant__ SegTable st, int split) {
+__global__ void __launch_bounds__(MC_THREADS, mc_ctas(CHROMA, SPLIT)) k_mc(const __grid_constant__ SegTable st, int split) {
     __shared__ uint2 s_pred[MC_STRIP_ROWS][MC_THREADS];   // list-0 predictions of bi strips
     const int tid = threadIdx.x;
     pdl_next();
