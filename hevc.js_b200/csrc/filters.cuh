@@ -13,9 +13,10 @@
 //      by plane and direction.
 //   2. vertical edges, 3. horizontal edges: one segment per thread, on 16-bit lanes.
 //   4. SAO on 16-bit lanes, 8 samples per thread and step, and the store.
-// Bound by instructions: 16 1080p P/B pictures issue 67 million warp instructions in 108 us, at
-// 0.58 per scheduler and cycle; their bytes take 19 us.  Before, as three kernels through memory
-// (vertical edges, horizontal edges, SAO), 93 million in 163 us.
+// Bound by instructions: 16 1080p P/B pictures issue 67 million warp instructions in 104 us, at
+// 0.6 per scheduler and cycle; their bytes take 19 us.  Before, as three kernels through memory
+// (vertical edges, horizontal edges, SAO), 93 million in 163 us.  No load is waited for where the
+// next one could be issued: 108 us with grid words and SAO records read one after the other.
 #pragma once
 
 #include "device_common.cuh"
@@ -310,8 +311,10 @@ __global__ void __launch_bounds__(THREADS, lf_ctas(THREADS)) k_loop_filter(const
 #pragma unroll 1
         for (int q = tid; q < LF_U * LF_U; q += THREADS) {
             const int ux = (x0 >> 2) - 1 + q % LF_U, uy = (y0 >> 2) - 1 + q / LF_U;
-            S.blk[q] = ux >= 0 && ux < gw && uy >= 0 && uy < H >> 2 ? __ldg(&P.blk[(int64_t)uy * gw + ux]) : 0u;
+            if (ux >= 0 && ux < gw && uy >= 0 && uy < H >> 2) cp_async4(S.blk + q, P.blk + (int64_t)uy * gw + ux);
+            else S.blk[q] = 0u;
         }
+        cp_async_commit();
         if (tid < 52) S.beta[tid] = c_beta[tid];
         if (tid < 54) S.tc[tid] = c_tc[tid];
         if (tid < 58) S.qpc[tid] = c_qpc[tid];
@@ -324,26 +327,6 @@ __global__ void __launch_bounds__(THREADS, lf_ctas(THREADS)) k_loop_filter(const
         if (tid == 99) S.slice = slice_at(P, 0);
     }
     const int cpt = lctb >= 6 ? 1 : LF_T >> lctb;   // CTBs across the tile
-    if (THREADS - 1 - tid < cpt * cpt * 3) {
-        const int ci = (THREADS - 1 - tid) % 3, k = (THREADS - 1 - tid) / 3;
-        const int cx = (x0 >> lctb) + k % cpt, cy = (y0 >> lctb) + k / cpt;
-        LfSao s = {0, 0, 0, 0, 0, 0};
-        if (P.sao_enabled && cx < P.wctb && cy < P.hctb) {
-            const hevc_sao_t& sp = P.sao[cy * P.wctb + cx];
-            s.type = sp.type[ci];
-            s.cls = sp.eo_class[ci];
-            if (s.type == 2) {   // the index computed is 4 - edgeIdx
-                const int pitch = ci ? LF_CP : LF_LP, dx = s.cls == 1 ? 0 : (s.cls == 3 ? 1 : -1), dy = s.cls == 0 ? 0 : -1;
-                s.a0 = (int16_t)(dy * pitch + dx);
-                for (int q = 0; q < 4; q++) s.lo |= (uint32_t)(uint8_t)sp.offset[ci][4 - q] << (8 * q);
-                s.hi = (uint8_t)sp.offset[ci][0];
-            } else {             // index 4 outside the four bands: no offset
-                s.k = (uint32_t)(uint16_t)(-(int)sp.band_pos[ci]) * 0x00010001u;
-                for (int q = 0; q < 4; q++) s.lo |= (uint32_t)(uint8_t)sp.offset[ci][q] << (8 * q);
-            }
-        }
-        S.sao[ci * LF_CTBS + k] = s;
-    }
     pdl_wait();
     // ---- the samples, in 16-byte pieces (one that starts inside the picture ends inside the
     // row's pitch, a multiple of 64): 6 of 8 threads per luma row, 4 per chroma row
@@ -366,7 +349,9 @@ __global__ void __launch_bounds__(THREADS, lf_ctas(THREADS)) k_loop_filter(const
             }
         }
     }
+    cp_async_commit();
     if (deblock) {
+        cp_async_wait<1>();
         __syncthreads();   // grid words, tables, counts
         // ---- 1. the segments to filter
         const bool boundaries = P.tiles_check || P.slice_check;
@@ -404,7 +389,35 @@ __global__ void __launch_bounds__(THREADS, lf_ctas(THREADS)) k_loop_filter(const
             lf_append(on && dir == 1, i, S.luma[1], &S.n_luma[1], lane);
         }
     }
-    cp_async_wait_all();
+    // SAO parameters, while the samples are on their way: a CTB and plane per thread, the record's
+    // bytes in one round of loads
+    if (THREADS - 1 - tid < cpt * cpt * 3) {
+        const int ci = (THREADS - 1 - tid) % 3, k = (THREADS - 1 - tid) / 3;
+        const int cx = (x0 >> lctb) + k % cpt, cy = (y0 >> lctb) + k / cpt;
+        LfSao s = {0, 0, 0, 0, 0, 0};
+        if (P.sao_enabled && cx < P.wctb && cy < P.hctb) {
+            const hevc_sao_t& sp = P.sao[cy * P.wctb + cx];
+            const int8_t* const off = sp.offset[ci];
+            const int band = sp.band_pos[ci];
+            s.type = sp.type[ci];
+            s.cls = sp.eo_class[ci];
+            s.lo = (uint8_t)off[0] | (uint32_t)(uint8_t)off[1] << 8 | (uint32_t)(uint8_t)off[2] << 16 |
+                   (uint32_t)(uint8_t)off[3] << 24;
+            s.hi = (uint8_t)off[4];
+            if (s.type == 2) {   // the index computed is 4 - edgeIdx
+                const int pitch = ci ? LF_CP : LF_LP, dx = s.cls == 1 ? 0 : (s.cls == 3 ? 1 : -1), dy = s.cls == 0 ? 0 : -1;
+                s.a0 = (int16_t)(dy * pitch + dx);
+                const uint32_t lo = s.lo;
+                s.lo = __byte_perm(lo, s.hi, 0x1234);
+                s.hi = lo & 0xFFu;
+            } else {             // index 4 outside the four bands: no offset
+                s.k = (uint32_t)(uint16_t)(-band) * 0x00010001u;
+                s.hi = 0u;
+            }
+        }
+        S.sao[ci * LF_CTBS + k] = s;
+    }
+    cp_async_wait<0>();
     __syncthreads();
     // ---- 2., 3. vertical, then horizontal edges.  A segment writes only words (luma) or samples
     // (chroma) that no other of its direction touches.  Chroma segments go to the last warps,
