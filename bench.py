@@ -693,8 +693,13 @@ def run_ours(args, hb, rank, world, local):
                                 "single_thread": {"value": round(n1 / t1, 3), "unit": "frames/s", "cores": 1,
                                                   "sample": f"{n1} pictures spread over the GOP work list on "
                                                             f"one thread ({t1:.1f} s)"}}
-        line["dropin"] = run_dropin()
-        line["dropin_generated"] = run_dropin_generated()
+        from hevc_b200.build import DROPIN_SO
+        if os.path.exists(DROPIN_SO):
+            line["dropin"] = run_dropin()
+            line["dropin_generated"] = run_dropin_generated()
+        else:   # a host without the reference's parser sources
+            why = f"{os.path.basename(DROPIN_SO)} is not built: it takes the reference's parser sources"
+            line["dropin"] = line["dropin_generated"] = {"unavailable": why}
     for st in gop_streams:
         st.close()
     if world > 1:
