@@ -1481,11 +1481,11 @@ struct Exec {
 
 // Warps per CTU of an intra launch (IC_WIDE or IC_NARROW).  Wide, two CTAs per SM, where the
 // chains of dependent TUs decide: a launch whose deepest picture has `depth` TUs in its
-// longest chain takes about 0.4 us a step.  Narrow, three CTAs per SM, where the number of
-// items does, 1.1 ns each on 148 SMs, and where a CTU has too few for 15 warps.  Measured
-// (us, wide / narrow): 1 and 8 1080p I pictures 482 / 583 and 580 / 687, with 32x32 and 16x16
-// CTBs (4 pictures) 511 / 557 and 854 / 748; 1, 4, 8 and 16 1080p P/B pictures 42 / 49,
-// 59 / 62, 89 / 83 and 142 / 126; 8 with 60 % intra CUs 359 / 415.
+// longest chain takes about 0.4 us a step.  Narrow, four CTAs per SM, where the number of
+// items does, 1.1 ns each on 148 SMs, and where a CTU has too few for 15 warps.  Measured with
+// the plan (us, wide / narrow): 1 and 8 1080p I pictures 498 / 644 and 594 / 757, with 32x32 and
+// 16x16 CTBs (4 pictures) 520 / 595 and 874 / 732; 1, 4, 6, 8 and 16 1080p P/B pictures 46 / 54,
+// 64 / 67, 75 / 75, 91 / 88 and 146 / 123; 8 with 60 % intra CUs 394 / 512.
 bool intra_wide(int ctus, int64_t items, int depth, int sms) {
     return items >= 16ll * ctus && (items >= 64ll * ctus || 400ll * depth >= items * 163 / sms);
 }

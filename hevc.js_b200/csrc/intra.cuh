@@ -527,7 +527,6 @@ struct IntraSmem {
     alignas(16) uint8_t tiles[IC_TILES + 16];   // and the constant 128, for TUs with no reference sample
     alignas(16) IntraTask task[IC_MAX_TUS];     // the CTU's part of PicDesc::itu_task
     alignas(16) int16_t res[IC_MAX_RES + 16];   // and the residual of 4x4 TUs without one
-    alignas(16) uint2 taps[36 * 2 * 16];        // c_intra_taps
     alignas(16) uint8_t edge[IC_EDGES];     // PicDesc::ictu_edge
     alignas(16) uint16_t rev[IC_DEP_STAGE + 2];   // the CTU's part of PicDesc::rev
     uint64_t bar[IC_MAX_TUS];               // what each TU waits for
@@ -539,7 +538,7 @@ struct IntraSmem {
 static_assert(IC_LH * IC_LP % 16 == 0 && IC_CH * IC_CP % 16 == 0, "the tiles' rows lie on 16-byte boundaries");
 
 template <int WARPS>
-__global__ void __launch_bounds__(32 * WARPS, 24 / WARPS + (WARPS > 8)) k_intra_ctus(const __grid_constant__ SegTable st,
+__global__ void __launch_bounds__(32 * WARPS, 32 / WARPS) k_intra_ctus(const __grid_constant__ SegTable st,
                                                                                  int32_t* tickets, int total,
                                                                                  uint32_t* sticky) {
     constexpr uint32_t FULL = 0xffffffffu;
@@ -548,9 +547,6 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS + (WARPS > 8)) k_intra_
     IntraSmem& S = *reinterpret_cast<IntraSmem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
     pdl_next();
-#pragma unroll 1
-    for (int q = tid; q < (int)sizeof(S.taps) / 16; q += THREADS)
-        cp_async16(reinterpret_cast<uint4*>(S.taps) + q, reinterpret_cast<const uint4*>(c_intra_taps.t) + q);
     pdl_wait();
     if (tid == 0) {
         // Each picture hands out its CTUs by ticket in wavefront order.  CTAs start at picture
@@ -743,7 +739,7 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS + (WARPS > 8)) k_intra_
             // the tile (IntraTaps); lane k finds where index k of the reference array lies.
             // No branch but DC's between the wait and the completion: one cost a lone warp
             // some 25 cycles.
-            const uint2 taps = S.taps[(task.mode * 2 + (chroma ? 1 : 0)) * 16 + (lane & 15)];
+            const uint2 taps = __ldg(reinterpret_cast<const uint2*>(c_intra_taps.t) + (task.mode * 2 + (chroma ? 1 : 0)) * 16 + (lane & 15));
             const int w = task_where(task, 4, pitch, plan_min(lane, 16));
             IntraTaps k = intra_taps_unpack(taps.x, taps.y);
             int at[4];
