@@ -1479,15 +1479,22 @@ struct Exec {
     int32_t* tickets() const { return reinterpret_cast<int32_t*>(static_cast<uint8_t*>(flow) + sizeof(FlowState) + 16); }
 };
 
-// Warps per CTU of an intra launch (IC_WIDE or IC_NARROW).  Wide, two CTAs per SM, where the
-// chains of dependent TUs decide: a launch whose deepest picture has `depth` TUs in its
-// longest chain takes about 0.4 us a step.  Narrow, four CTAs per SM, where the number of
-// items does, 1.1 ns each on 148 SMs, and where a CTU has too few for 15 warps.  Measured with
-// the plan (us, wide / narrow): 1 and 8 1080p I pictures 498 / 644 and 594 / 757, with 32x32 and
-// 16x16 CTBs (4 pictures) 520 / 595 and 874 / 732; 1, 4, 6, 8 and 16 1080p P/B pictures 46 / 54,
-// 64 / 67, 75 / 75, 91 / 88 and 146 / 123; 8 with 60 % intra CUs 394 / 512.
-bool intra_wide(int ctus, int64_t items, int depth, int sms) {
-    return items >= 16ll * ctus && (items >= 64ll * ctus || 400ll * depth >= items * 163 / sms);
+// Warps per CTU of an intra launch.  Where the chains of dependent TUs decide, more warps: a launch
+// whose deepest picture has `depth` TUs in its longest chain takes about 0.4 us a step.  Fewer,
+// and more CTAs per SM, where the number of items does, 1.1 ns each on 148 SMs, and where a CTU
+// has too few for its warps.  IC_FULL, one CTA per SM, when the chain takes twice as long as the
+// items do and the picture it belongs to has 64 items a CTU (CTUs of 64x64 full of intra TUs);
+// IC_WIDE, two, while it takes longer; else IC_NARROW, four.  Measured with the plan (us, full /
+// wide / narrow): 1, 4 and 8 1080p I pictures 420 / 498 / 644, 461 / 523 and 597 / 594 / 757, 4 with
+// 32x32 and 16x16 CTBs 572 / 520 / 595 and 1,330 / 874 / 732; 4 and 16 720p I pictures 295 / 339
+// and 487 / 435; 1 and 4 2160p 871 / 1,014 and 1,170 / 1,158; 1, 4, 6, 8 and 16 1080p P/B pictures
+// 43 / 46 / 54, 75 / 64 / 67, 93 / 75 / 75, 119 / 91 / 88 and 205 / 146 / 123; 8 with 60 % intra CUs
+// 387 / 394 / 512.
+// deep_ctus, deep_items: of the deepest picture.
+int intra_warps(int ctus, int64_t items, int depth, int deep_ctus, int64_t deep_items, int sms) {
+    const int64_t chain = 400ll * depth, work = items * 163 / sms;
+    if (deep_items >= 64ll * deep_ctus && chain >= 2 * work) return IC_FULL;
+    return items >= 16ll * ctus && (items >= 64ll * ctus || chain >= work) ? IC_WIDE : IC_NARROW;
 }
 
 // The intra launches of a batch, one per group of up to MAX_SEGS pictures: CTAs take intra CTUs
@@ -1496,14 +1503,14 @@ bool intra_wide(int ctus, int64_t items, int depth, int sms) {
 struct IntraLaunch {
     SegTable t;
     int total;
-    bool wide;
+    int warps;
 };
 int intra_launches(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n, std::vector<IntraLaunch>& out) {
     for (int k = 0; k < n;) {
         IntraLaunch g;
         std::memset(&g.t, 0, sizeof(g.t));
-        int total = 0, depth = 0;
-        int64_t items = 0;
+        int total = 0, depth = 0, deep_ctus = 0;
+        int64_t items = 0, deep_items = 0;
         for (; k < n && g.t.n < MAX_SEGS; k++) {
             hevcgpu_job* j = jobs[k];
             if (j->n_ictu == 0) continue;
@@ -1520,11 +1527,15 @@ int intra_launches(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, i
             sg.aux1 = ++j->epoch;
             total += j->n_ictu;
             items += j->n_items;
-            depth = std::max(depth, j->depth);
+            if (j->depth > depth) {
+                depth = j->depth;
+                deep_ctus = j->n_ictu;
+                deep_items = j->n_items;
+            }
         }
         if (g.t.n == 0) continue;
         g.total = total;
-        g.wide = intra_wide(total, items, depth, ctx->sm_count);
+        g.warps = intra_warps(total, items, depth, deep_ctus, deep_items, ctx->sm_count);
         out.push_back(g);
     }
     return HEVCGPU_OK;
@@ -1583,10 +1594,9 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
     for (const IntraLaunch& g : intra) {
         StageMark m(ctx, ex.stream, 3);
         if (&g != &intra[0] && (rc = plan(g, true))) return rc;
-        rc = g.wide ? L.go_smem(k_intra_ctus<IC_WIDE>, dim3(g.total), dim3(32 * IC_WIDE), sizeof(IntraSmem), g.t, ex.tickets(),
-                                g.total, sticky)
-                    : L.go_smem(k_intra_ctus<IC_NARROW>, dim3(g.total), dim3(32 * IC_NARROW), sizeof(IntraSmem), g.t,
-                                ex.tickets(), g.total, sticky);
+        auto* const kernel = g.warps == IC_FULL ? k_intra_ctus<IC_FULL>
+                             : g.warps == IC_WIDE ? k_intra_ctus<IC_WIDE> : k_intra_ctus<IC_NARROW>;
+        rc = L.go_smem(kernel, dim3(g.total), dim3(32 * g.warps), sizeof(IntraSmem), g.t, ex.tickets(), g.total, sticky);
         if (rc) return rc;
     }
     if (stages & ST_SAO) {   // deblocking, when asked for, then SAO into the slot
@@ -1678,10 +1688,8 @@ int hevcgpu_create(int device, hevcgpu_ctx_t** out) {
         return fail(HEVCGPU_EUNSUPPORTED, "device %d is sm_%d%d; this library is built for sm_100a", device,
                     prop.major, prop.minor);
     CUDA_TRY(cudaSetDevice(device));
-    CUDA_TRY(cudaFuncSetAttribute(k_intra_ctus<IC_NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(IntraSmem)));
-    CUDA_TRY(cudaFuncSetAttribute(k_intra_ctus<IC_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(IntraSmem)));
+    for (auto* k : {k_intra_ctus<IC_NARROW>, k_intra_ctus<IC_WIDE>, k_intra_ctus<IC_FULL>})
+        CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(IntraSmem)));
     for (auto* k : {k_loop_filter<128>, k_loop_filter<256>})
         CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lf_pad(1, 128)));
     auto* c = new (std::nothrow) hevcgpu_ctx();

@@ -231,9 +231,9 @@ __device__ __forceinline__ void intra_predict(const IntraTask& task, int strong_
 // watcher: it alone polls words of other CTUs, so the workers only read shared memory and
 // wait on shared-memory barriers, which suspend them without taking issue slots.
 // ---------------------------------------------------------------------------------------
-// Warps of a CTA (the last one watches): IC_WIDE where the chains decide, IC_NARROW where the
-// number of CTUs does (intra_wide).
-constexpr int IC_NARROW = 8, IC_WIDE = 16;
+// Warps of a CTA (the last one watches): the more, the more the chains decide and not the number
+// of TUs (intra_warps).
+constexpr int IC_NARROW = 8, IC_WIDE = 16, IC_FULL = 24;
 // Tiles: a margin of 16 bytes (its last byte is the column left of the CTU; 16 keeps the
 // CTU's rows on 16-byte boundaries for the asynchronous copies), the CTU, the CTU to the
 // right (row -1 only); row -1 first.  Pitches that are odd multiples of 16 spread a column
@@ -531,7 +531,7 @@ struct IntraSmem {
     alignas(16) uint16_t rev[IC_DEP_STAGE + 2];   // the CTU's part of PicDesc::rev
     uint64_t bar[IC_MAX_TUS];               // what each TU waits for
     uint2 watch[IC_MAX_WATCH];              // PicDesc::watch_plan, y counted down as border words come
-    IntraWarpSmem ws[IC_WIDE - 1];
+    IntraWarpSmem ws[IC_FULL - 1];
     int ticket, pic_index, next;
     volatile int abort;
 };
