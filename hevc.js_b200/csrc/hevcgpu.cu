@@ -1485,11 +1485,11 @@ struct Exec {
 // has too few for its warps.  IC_FULL, one CTA per SM, when the chain takes twice as long as the
 // items do and the picture it belongs to has 64 items a CTU (CTUs of 64x64 full of intra TUs), or
 // four times as long and it has 32, or 16 and two CTUs per SM at most; IC_WIDE, two, while it
-// takes longer; else IC_NARROW, four.  Measured with the plan (us, full / wide / narrow): 1, 4 and 8
+// takes longer; else IC_NARROW, three.  Measured with the plan (us, full / wide / narrow): 1, 4 and 8
 // 1080p I pictures 420 / 498 / 644, 461 / 523 and 597 / 594 / 757, 4 with 32x32 and 16x16 CTBs 572 /
-// 520 / 595 and 1,330 / 874 / 732; 4 and 16 720p I pictures 295 / 339 and 487 / 435; 1 and 4 2160p
-// 871 / 1,014 and 1,170 / 1,158; 1, 4, 6, 8 and 16 1080p P/B pictures 43 / 46 / 54, 75 / 64 / 67,
-// 93 / 75 / 75, 119 / 91 / 88 and 205 / 146 / 123; 8 with 60 % intra CUs 387 / 394 / 512.  Full /
+// 520 / 595 and 1,330 / 874 / 750; 4 and 16 720p I pictures 295 / 339 and 487 / 435; 1 and 4 2160p
+// 871 / 1,014 and 1,170 / 1,158; 1, 4, 8 and 16 1080p P/B pictures 43 / 46 / 54, 75 / 64 / 67,
+// 119 / 91 / 91 and 205 / 146 / 129; 8 with 60 % intra CUs 387 / 394 / 512.  Full /
 // wide: one and two 1080p I pictures with 32x32 CTBs 425 / 466 and 435 / 478, one 416x240, 832x480
 // and 1280x720 P/B picture 23 / 25, 44 / 48 and 41 / 44; but one 1000x568 with 32x32 CTBs (363 CTUs of
 // 19 items) 41 / 38.

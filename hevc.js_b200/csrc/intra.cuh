@@ -28,8 +28,8 @@
 //     side;
 //   - the code is small: what does not run per TU is a kernel of its own, since instruction
 //     cache misses were half of all stalls with it inside.
-// 8 1080p I pictures: 0.58 ms, 2.18 with waits on every owner and the work after the wait; 1 and
-// 16 1080p P/B pictures 43 and 126 us, 107 and 276 then.
+// With the plan, 1 and 8 1080p I pictures take 0.42 and 0.59 ms (the eight 2.18 with waits on every
+// owner and the work after the wait), 1 and 16 1080p P/B pictures 43 and 129 us, 107 and 276 then.
 #pragma once
 
 #include <cuda/atomic>
@@ -537,8 +537,13 @@ struct IntraSmem {
 };
 static_assert(IC_LH * IC_LP % 16 == 0 && IC_CH * IC_CP % 16 == 0, "the tiles' rows lie on 16-byte boundaries");
 
+// CTAs per SM that the register budget is sized for.  Four narrow ones take the register file whole:
+// a batch of 16 1080p P/B pictures alone 393 us instead of 398, but on two lanes, whose kernels
+// share the SMs, 38,000 frames/s instead of 42,400.
+constexpr int ic_ctas(int warps) { return warps == IC_NARROW ? 3 : 32 / warps; }
+
 template <int WARPS>
-__global__ void __launch_bounds__(32 * WARPS, 32 / WARPS) k_intra_ctus(const __grid_constant__ SegTable st,
+__global__ void __launch_bounds__(32 * WARPS, ic_ctas(WARPS)) k_intra_ctus(const __grid_constant__ SegTable st,
                                                                                  int32_t* tickets, int total,
                                                                                  uint32_t* sticky) {
     constexpr uint32_t FULL = 0xffffffffu;
