@@ -560,7 +560,7 @@ def run_ours(args, hb, rank, world, local):
     # --warmup 0 --streams 2), scaled by 4 to 8 pictures per launch (each picture is
     # independent work), the GOP's total divided by its 60 batches; taken again whenever the
     # stage's kernels change
-    ncu_dram_gop8 = {"mc": 57564587, "residual": 83248384, "intra": 26987537}
+    ncu_dram_gop8 = {"mc": 59200734, "residual": 47180459, "intra": 30119697, "loop_filter": 37424230}
     traffic = (ncu_dram_gop8[dom] if dom in ncu_dram_gop8 and (W, H, G, F) == (W_DEFAULT, H_DEFAULT, 8, 60)
                else None)
 
