@@ -166,7 +166,7 @@ struct Seg {
     const PicDesc* pic;
     int32_t n_items;
     int32_t block0;
-    int32_t aux0, aux1;   // per-launch extras (intra arming: queue offsets)
+    int32_t aux0, aux1;   // per-launch extras (aux1 of an intra launch: its epoch)
 };
 struct SegTable {
     int32_t n;
