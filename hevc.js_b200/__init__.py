@@ -251,6 +251,7 @@ def gpu_lib():
                                              C.POINTER(C.c_uint16), C.POINTER(C.c_uint16), C.c_int32], C.c_int),
             "hevcgpu_slot_checksum": ([P, C.c_int32, C.POINTER(abi.Crop), C.POINTER(C.c_uint32)], C.c_int),
             "hevcgpu_intra_schedule": ([P, C.POINTER(abi.IntraSchedule)], C.c_int),
+            "hevcgpu_intra_levels": ([P, C.POINTER(C.POINTER(C.c_int32)), C.POINTER(C.c_int32)], C.c_int),
             "hevcgpu_mc_strips": ([P, C.POINTER(C.POINTER(C.c_uint32)), C.POINTER(C.c_int32),
                                    C.POINTER(C.POINTER(C.c_uint32)), C.POINTER(C.c_int32)], C.c_int),
             "hevcgpu_slot_device_ptr": ([P, C.c_int32, C.POINTER(P), C.POINTER(P), C.POINTER(P),
@@ -587,6 +588,16 @@ def intra_schedule(pic):
             "task_tu": arr(out.task_tu, out.n_task, np.int64), "task_deps": arr(out.task_deps, out.n_task, np.uint32),
             "deps": arr(out.deps, out.n_dep, np.uint32), "task_flags": arr(out.task_flags, out.n_task, np.uint8),
             "ctu_watch": arr(out.ctu_watch, out.n_ctu, np.uint32), "watch": arr(out.watch, out.n_watch, np.int64)}
+
+
+def intra_levels(pic):
+    """The order of a picture whose intra TUs the back end does level by level
+    (hevcgpu_intra_levels; host work only): (TU index, items to be complete before) per work item,
+    empty for pictures that are done CTU by CTU."""
+    lib = gpu_lib()
+    p, n = C.POINTER(C.c_int32)(), C.c_int32(0)
+    _check(lib.hevcgpu_intra_levels(C.cast(pic.syn_ptr, C.c_void_p), C.byref(p), C.byref(n)))
+    return np.ctypeslib.as_array(p, shape=(n.value, 2)).copy() if n.value > 0 else np.zeros((0, 2), np.int32)
 
 
 def mc_strips(pic):

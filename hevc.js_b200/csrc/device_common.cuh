@@ -43,6 +43,9 @@ constexpr uint8_t ITU_PUBLISH = 1u;
 constexpr int IC_BAND = 8;
 __host__ __device__ constexpr int intra_bands(int log2) { return log2 > 3 ? (1 << log2) / IC_BAND : 1; }
 
+constexpr int IL_BAND_SHIFT = 24, IL_TASK = (1 << IL_BAND_SHIFT) - 1;   // of PicDesc::level_task
+constexpr int IL_DONE = 64, IL_STATE = IL_DONE + 1;   // words of PicDesc::level_state: taken (0), complete (in another line)
+
 // An intra CTU: its raster address, its TUs in the task order arrays, its entries in the
 // dependency lists and the watch list, its residuals in the residual buffer, its work items,
 // and which neighbour CTUs its TUs may read (NB_*).  Three 16-byte loads.
@@ -108,6 +111,11 @@ struct PicDesc {
     uint16_t* rev;
     uint8_t* ictu_edge;
     uint64_t* edge;                      // border words of every CTU, 1 << log2_ctb each
+    // or, in a picture that k_intra_levels does: its work items in the order they are taken, task
+    // index | band << IL_BAND_SHIFT, and the number of items in the levels before; items taken,
+    // items complete
+    const int2* level_task;
+    int32_t* level_state;
     int32_t num_pus;
     int32_t num_slices;
     int32_t log2_ctb, wctb, hctb;

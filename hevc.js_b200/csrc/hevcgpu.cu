@@ -22,6 +22,7 @@
 
 #include "hevcgpu.h"
 #include "intra.cuh"
+#include "intra_levels.cuh"
 #include "mc.cuh"
 #include "kernels.cuh"
 #include "filters.cuh"
@@ -427,6 +428,7 @@ struct hevcgpu_job {
     int32_t depth = 0;                  // TUs of the longest dependency chain
     const IntraCtu* d_ictu = nullptr;   // their records
     size_t edge_bytes = 0;              // border words of the intra stage (PicDesc::edge)
+    int32_t n_level_items = 0;          // work items of a picture that k_intra_levels does, else 0
     uint32_t spare_dep = 0;             // dependency list entry kept for the planted wait
     int32_t epoch = 0;                  // intra launches of this job so far
     int32_t n_pus = 0;
@@ -615,6 +617,11 @@ struct BuildScratch {
     std::vector<IntraCtu> ictu;
     std::vector<uint32_t> watch_geo;
     std::vector<uint16_t> items;
+    // A picture that k_intra_levels does, its TUs level by level (PicDesc::level_task), and per 4x4
+    // unit the levels up to its last writer and its last reader.
+    bool by_levels = false;
+    std::vector<int2> level_task;
+    std::vector<int32_t> level_of, written[3], read[3];
     // intra schedule
     std::vector<int32_t> dep_at, deps, pos, cnt;
     std::vector<std::pair<int64_t, int32_t>> runs;   // (wavefront key, first TU) of each CTU's run
@@ -757,7 +764,10 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
     itu_dep.clear();
     dep_out.clear();
     BS.depth = 0;
+    BS.by_levels = false;
     if (!n_intra) return HEVCGPU_OK;
+    bool larger = false;   // than its CTB
+    uint32_t twice = 0;    // a unit that an earlier TU owns already
     auto& level = BS.level;
     auto& ctu_of = BS.ctu_of;
     auto& dep_at = BS.dep_at;       // decode order: first entry of TU b's owners in deps
@@ -847,11 +857,16 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
         level[(size_t)b] = dp;
         BS.depth = std::max(BS.depth, dp + 1);
         const uint32_t mark = gtag | (uint32_t)b;
+        larger |= n * sub > ctb;
         for (int y = uy; y < uy + n / 4; y++) {
             uint32_t* r = own + (size_t)y * row;
-            for (int x = ux; x < ux + n / 4; x++) r[x] = mark;
+            for (int x = ux; x < ux + n / 4; x++) {
+                twice |= (uint32_t)((r[x] & GEN_BITS) == gtag);
+                r[x] = mark;
+            }
         }
     }
+    BS.by_levels = larger || twice;
     dep_at[(size_t)n_intra] = (int32_t)n_own;
     deps.resize(n_own);
     // Task order: CTUs in wavefront order (key 2 * row + column, then raster), each
@@ -1020,6 +1035,54 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
     return HEVCGPU_OK;
 }
 
+// The levels of a picture that k_intra_levels does, from its schedule: a TU comes after the TUs
+// before it in decode order that write a sample it reads (or could: availability is not looked at)
+// or covers, and after those that read a sample it covers.
+void build_intra_levels(BuildScratch& BS, const hevc_picture_syntax_t* s) {
+    const size_t n_tu = BS.itu_rec.size();
+    for (int c = 0; c < 3; c++) {
+        const size_t units = (size_t)((s->params.width >> (c ? 1 : 0)) / 4) * (size_t)((s->params.height >> (c ? 1 : 0)) / 4);
+        BS.written[c].assign(units, 0);
+        BS.read[c].assign(units, 0);
+    }
+    auto& level = BS.level_of;   // in decode order
+    level.resize(n_tu);
+    int levels = 0;
+    for (size_t b = 0; b < n_tu; b++) {
+        const hevc_tu_t& t = s->tus[BS.intra_list[b]];
+        const int c = t.c_idx, uw = (s->params.width >> (c ? 1 : 0)) / 4, uh = (s->params.height >> (c ? 1 : 0)) / 4;
+        const int ux = t.x / 4, uy = t.y / 4, nu = (1 << t.log2_size) / 4;
+        int32_t* const written = BS.written[c].data();
+        int32_t* const read = BS.read[c].data();
+        auto around = [&](auto&& f) {
+            for (int x = std::max(0, ux - 1); uy > 0 && x < std::min(uw, ux + 2 * nu); x++) f((size_t)(uy - 1) * uw + x);
+            for (int y = uy; ux > 0 && y < std::min(uh, uy + 2 * nu); y++) f((size_t)y * uw + ux - 1);
+        };
+        auto covered = [&](auto&& f) {
+            for (int y = uy; y < uy + nu; y++)
+                for (int x = ux; x < ux + nu; x++) f((size_t)y * uw + x);
+        };
+        int l = 0;
+        around([&](size_t u) { l = std::max(l, written[u]); });
+        covered([&](size_t u) { l = std::max({l, written[u], read[u]}); });
+        level[b] = l++;
+        around([&](size_t u) { read[u] = std::max(read[u], l); });
+        covered([&](size_t u) { written[u] = l; });
+        levels = std::max(levels, l);
+    }
+    auto& first = BS.cnt;   // of each level
+    auto bands = [&](size_t b) { return intra_bands(s->tus[BS.intra_list[b]].log2_size); };
+    first.assign((size_t)levels + 1, 0);
+    for (size_t b = 0; b < n_tu; b++) first[(size_t)level[b] + 1] += bands(b);
+    for (int l = 0; l < levels; l++) first[(size_t)l + 1] += first[(size_t)l];
+    BS.level_task.resize((size_t)first[(size_t)levels]);
+    std::vector<int32_t> fill(first.begin(), first.end());
+    for (size_t b = 0; b < n_tu; b++)
+        for (int k = 0; k < bands(b); k++)
+            BS.level_task[(size_t)fill[(size_t)level[b]]++] =
+                make_int2(BS.pos[b] | k << IL_BAND_SHIFT, first[(size_t)level[b]]);
+}
+
 // The caller's large arrays (PUs, 4x4 grid, TUs, coefficient levels) have their own device
 // buffer and are uploaded first, so that the transfer overlaps the building of the work
 // lists: straight from where they lie when they are in page-locked memory, else through
@@ -1154,6 +1217,14 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     auto& itu_dep = BS.itu_dep;         // per task entry: (dependency list offset << 6) | count
     auto& dep_out = BS.dep_out;         // dependency lists in task order
     if ((rc = build_intra_schedule(BS, s, &j->spare_dep))) return rc;
+    BS.level_task.clear();
+    if (BS.by_levels) {   // no CTU of it goes to k_intra_ctus
+        build_intra_levels(BS, s);
+        ictu.clear();
+        BS.items.clear();
+        BS.watch_geo.clear();
+    }
+    j->n_level_items = (int32_t)BS.level_task.size();
     j->n_ictu = (int32_t)ictu.size();
     j->n_items = (int32_t)BS.items.size();
     j->depth = BS.depth;
@@ -1169,7 +1240,7 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     }
     j->n_pus = s->num_pus;
 
-    size_t o_wp, o_sao, o_sl, o_ti, o_slices, o_res, o_mc[2], o_ia, o_idp, o_itu, o_iro, o_dl, o_wl, o_it;
+    size_t o_wp, o_sao, o_sl, o_ti, o_slices, o_res, o_mc[2], o_ia, o_idp, o_itu, o_iro, o_dl, o_wl, o_it, o_lt;
     size_t o_scal = 0;
     hevc_slice_t dflt{0, 0, 0, 1};
     const bool scaled = s->scaling && (stages & (ST_RESID | ST_INTRA));
@@ -1190,6 +1261,7 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
         o_dl = pk.add(dep_out.data(), sizeof(uint32_t) * dep_out.size());
         o_it = pk.add(BS.items.data(), sizeof(uint16_t) * BS.items.size());
         o_wl = pk.add(BS.watch_geo.data(), sizeof(uint32_t) * BS.watch_geo.size());
+        o_lt = pk.add(BS.level_task.data(), sizeof(int2) * BS.level_task.size());
     };
     Packer measure;
     pack(measure);
@@ -1207,13 +1279,14 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     size_t resid_bytes = j->has_intra ? sizeof(int16_t) * (size_t)align_up((int64_t)BS.res_total, 128) : 0;
     size_t mot_bytes = (stages & ST_DEBLOCK) ? sizeof(MotionEnt) * (size_t)align_up((int64_t)gw * gh, 32) : 0;
     // border words of the intra stage, then its plan
-    j->edge_bytes = j->has_intra ? sizeof(uint64_t) * (size_t)nctb * ctb : 0;
+    j->edge_bytes = j->n_ictu ? sizeof(uint64_t) * (size_t)nctb * ctb : 0;
     Packer plan;
     plan.size = resid_bytes + mot_bytes + j->edge_bytes;
     size_t o_task = 0, o_wplan = 0, o_rev = 0, o_edge = 0;
-    if (j->has_intra) {
+    const size_t o_state = plan.add(nullptr, j->n_level_items ? IL_STATE * sizeof(int32_t) : 0);
+    if (j->n_ictu) {
         o_task = plan.add(nullptr, sizeof(IntraTask) * BS.items.size());
-        o_wplan = plan.add(nullptr, sizeof(uint2) * BS.watch.size());
+        o_wplan = plan.add(nullptr, sizeof(uint2) * BS.watch_geo.size());
         o_rev = plan.add(nullptr, sizeof(uint16_t) * (dep_out.size() + 2));
         o_edge = plan.add(nullptr, (size_t)IC_EDGES * ictu.size());
     }
@@ -1256,6 +1329,8 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     D.watch_plan = reinterpret_cast<uint2*>(scratch + o_wplan);
     D.rev = reinterpret_cast<uint16_t*>(scratch + o_rev);
     D.ictu_edge = scratch + o_edge;
+    D.level_task = reinterpret_cast<const int2*>(base + o_lt);
+    D.level_state = reinterpret_cast<int32_t*>(scratch + o_state);
     // border words start below every epoch a launch can use
     if (j->edge_bytes && (rc = up({UploadOp::ZERO, D.edge, nullptr, j->edge_bytes}))) return rc;
     D.num_pus = s->num_pus;
@@ -1603,6 +1678,22 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
                              : g.warps == IC_WIDE ? k_intra_ctus<IC_WIDE> : k_intra_ctus<IC_NARROW>;
         rc = L.go_smem(kernel, dim3(g.total), dim3(32 * g.warps), sizeof(IntraSmem), g.t, ex.tickets(), g.total, sticky);
         if (rc) return rc;
+    }
+    for (int k = 0; (stages & ST_INTRA) && k < n;) {   // pictures done level by level
+        if (!jobs[k]->n_level_items) {
+            k++;
+            continue;
+        }
+        StageMark m(ctx, ex.stream, 3);
+        SegTable t;
+        std::memset(&t, 0, sizeof(t));
+        for (; k < n && t.n < MAX_SEGS; k++) {
+            if (!jobs[k]->n_level_items) continue;
+            CUDA_TRY(cudaMemsetAsync(jobs[k]->host_desc.level_state, 0, IL_STATE * sizeof(int32_t), ex.stream));
+            t.s[t.n].pic = jobs[k]->d_desc;
+            t.s[t.n++].n_items = jobs[k]->n_level_items;
+        }
+        if ((rc = L.go(k_intra_levels, dim3(IL_CTAS, t.n), dim3(32 * IL_WARPS), t, sticky))) return rc;
     }
     if (stages & ST_SAO) {   // deblocking, when asked for, then SAO into the slot
         StageMark m(ctx, ex.stream, stages & ST_DEBLOCK ? 4 : 6);
@@ -2250,6 +2341,21 @@ int hevcgpu_intra_schedule(const hevc_picture_syntax_t* syn, hevc_intra_schedule
     return HEVCGPU_OK;
 }
 
+int hevcgpu_intra_levels(const hevc_picture_syntax_t* syn, const int32_t** order, int32_t* n) {
+    if (!order || !n) return fail(HEVCGPU_EINVAL, "null out");
+    *order = nullptr;
+    *n = 0;
+    hevc_intra_schedule_t sch;
+    if (int rc = hevcgpu_intra_schedule(syn, &sch)) return rc;
+    BuildScratch& BS = t_build;
+    if (!BS.by_levels) return HEVCGPU_OK;
+    build_intra_levels(BS, syn);
+    for (int2& e : BS.level_task) e.x = BS.itu[(size_t)(e.x & IL_TASK)];
+    *order = &BS.level_task[0].x;
+    *n = (int32_t)BS.level_task.size();
+    return HEVCGPU_OK;
+}
+
 int hevcgpu_mc_strips(const hevc_picture_syntax_t* syn, const uint32_t** luma, int32_t* n_luma,
                       const uint32_t** chroma, int32_t* n_chroma) {
     if (!luma || !n_luma || !chroma || !n_chroma) return fail(HEVCGPU_EINVAL, "null out");
@@ -2270,9 +2376,16 @@ int hevcgpu_mc_strips(const hevc_picture_syntax_t* syn, const uint32_t** luma, i
 
 int hevcgpu_job_plant_unmet_wait(hevcgpu_job_t* job) {
     if (!job) return fail(HEVCGPU_EINVAL, "null job");
-    if (job->n_ictu <= 0) return fail(HEVCGPU_EINVAL, "the job has no intra CTU to plant a wait in");
+    if (job->n_ictu <= 0 && !job->n_level_items) return fail(HEVCGPU_EINVAL, "the job has no intra CTU to plant a wait in");
     int rc = check_ctx(job->ctx);
     if (rc) return rc;
+    if (job->n_level_items) {   // the first item taken waits for more than there are
+        const int32_t never = INT32_MAX;
+        CUDA_TRY(cudaMemcpyAsync(const_cast<int32_t*>(&job->host_desc.level_task[0].y), &never, sizeof(never),
+                                 cudaMemcpyHostToDevice, job->ctx->stream));
+        CUDA_TRY(cudaStreamSynchronize(job->ctx->stream));
+        return HEVCGPU_OK;
+    }
     // Task 0 (the first TU of the first intra CTU) depends on nothing.  Its dependency list
     // now is the job's spare entry: an external dependency on its own completion, which only
     // it could publish.

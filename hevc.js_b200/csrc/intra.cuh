@@ -246,6 +246,10 @@ constexpr int IC_MAX_RES = 64 * 64 + 2 * 32 * 32;    // residual samples of a 64
 constexpr int IC_DEP_STAGE = 2048;                   // dependency entries staged per CTU
 constexpr int IC_MAX_WATCH = 128;                    // TUs of other CTUs a CTU waits for
 constexpr int IC_SOURCES = IC_MAX_TUS + IC_MAX_WATCH;   // what a TU can wait for: TUs here, watched TUs
+// These hold because intra TUs cover no sample twice and lie within their CTB (pictures for which
+// that is not so go to k_intra_levels): a work item covers a 4x4 unit or more, and a TU of u x u
+// units has at most 4u + 1 owners around it, five a unit at most.
+static_assert(5 * IC_MAX_TUS <= IC_DEP_STAGE, "a CTU's dependency entries fit");
 // Border words (4 samples) a CTU's TUs can read, per plane: the corner, the row above over two
 // CTUs, the column to the left.
 constexpr int IC_EDGE_L = 1 + 3 * 16, IC_EDGE_C = 1 + 3 * 8;

@@ -402,6 +402,15 @@ typedef struct hevc_intra_schedule {
 } hevc_intra_schedule_t;
 int  hevcgpu_intra_schedule(const hevc_picture_syntax_t* syn, hevc_intra_schedule_t* out);
 
+/* The order of a picture whose intra TUs cover samples twice or are larger than their CTB,
+ * which no bitstream that codes every block once gives: it is not done CTU by CTU but level
+ * by level, in decode order where that matters.  order holds two words per work item (a TU, or
+ * 8 rows of a larger one) in the order they are taken: the TU's index into syn->tus, and how
+ * many of the items before it must be complete first (all of the levels before its own).  *n
+ * is the number of items, 0 for every other picture.  Host work only; the array belongs to the calling thread and stays valid
+ * until its next call. */
+int  hevcgpu_intra_levels(const hevc_picture_syntax_t* syn, const int32_t** order, int32_t* n);
+
 /* The motion-compensation work lists the back end builds for a picture (no counterpart in
  * the reference; host work only), for tools and tests: one item per strip of 4 columns and
  * up to 16 rows of one PU in one plane, luma and chroma lists.  Item bits: 0-19 the PU,
