@@ -421,6 +421,7 @@ struct hevcgpu_job {
     PicDesc host_desc{};
     int32_t n_res[4] = {0, 0, 0, 0};
     const int32_t* d_res = nullptr;   // 32x32 first, then 16x16, 8x8, 4x4
+    bool res_by_size = false;         // TUs that cover each other's samples: a launch per size
     int32_t n_mc[2] = {0, 0};            // luma strips, chroma strips (mc.cuh items)
     const uint32_t* d_mc[2] = {nullptr, nullptr};
     int32_t n_ictu = 0;                 // CTUs that hold intra TUs
@@ -605,6 +606,7 @@ enum StageMask : int {
 // and no first-touch page faults per picture.
 struct BuildScratch {
     std::vector<int32_t> bins[4], intra_list, itu, level, ctu_of, order;
+    std::vector<uint8_t> coded[3];   // 4x4 units that coded inter TUs cover, a bit each (mark_block)
     // intra owner maps, one word per 4x4 unit: (generation << 24) | decode-order index of the
     // intra TU.  An entry is valid when its generation is this picture's, so the maps need
     // clearing only when the 8-bit generation wraps.
@@ -701,6 +703,20 @@ void build_mc_strips(BuildScratch& BS, const hevc_picture_syntax_t* s, int pitch
             }
         }
     }
+}
+
+// Marks the 4x4 units of a block in a plane's bit map, rows of `pitch` bytes; true if some were
+// marked already.  A block lies at a multiple of its size, so its units in a row share a byte.
+inline bool mark_block(uint8_t* map, int pitch, const hevc_tu_t& t) {
+    const int nu = (1 << t.log2_size) / 4, ux = t.x / 4;
+    const uint8_t units = (uint8_t)(((1u << nu) - 1u) << (ux & 7));
+    uint8_t* r = map + (size_t)(t.y / 4) * pitch + (ux >> 3);
+    uint8_t hit = 0;
+    for (int k = 0; k < nu; k++, r += pitch) {
+        hit |= *r & units;
+        *r |= units;
+    }
+    return hit != 0;
 }
 
 // Issue one queued CUDA call of a job's preparation on the context stream.
@@ -1194,12 +1210,20 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     intra_list.clear();
     for (auto& v : bins) v.reserve((size_t)s->num_tus / 2);
     intra_list.reserve((size_t)s->num_tus);
+    bool twice = false;   // two coded inter TUs cover a unit
+    const int map_pitch[2] = {(gw + 7) / 8, (gw / 2 + 7) / 8};
+    if (stages & ST_RESID)
+        for (int c = 0; c < 3; c++) BS.coded[c].assign((size_t)map_pitch[c ? 1 : 0] * (size_t)(c ? gh / 2 : gh), 0);
     for (int i = 0; i < s->num_tus; i++) {
         const hevc_tu_t& t = s->tus[i];
         bool intra = t.flags & HEVC_TU_INTRA;
-        if ((t.flags & HEVC_TU_CODED) && !intra && (stages & ST_RESID)) bins[t.log2_size - 2].push_back(i);
+        if ((t.flags & HEVC_TU_CODED) && !intra && (stages & ST_RESID)) {
+            bins[t.log2_size - 2].push_back(i);
+            twice |= mark_block(BS.coded[t.c_idx].data(), map_pitch[t.c_idx ? 1 : 0], t);
+        }
         if (intra && (stages & ST_INTRA)) intra_list.push_back(i);
     }
+    j->res_by_size = twice;
     j->has_intra = !intra_list.empty();
     // Intra schedule.  Per plane an owner map at 4-sample granularity records the latest
     // intra TU written there; intra TU B reads the units of its reference row
@@ -1498,18 +1522,30 @@ size_t lf_pad(int per_sm, int threads) {
 }
 
 // Adds a picture's coded TUs (items: by size, largest first) to a residual launch of `blocks`
-// CTAs so far; returns the new number.
-int res_add(ResTable& t, int blocks, const int32_t* items, const PicDesc* pic, const int32_t (&n)[4]) {
-    if (n[0] + n[1] + n[2] + n[3] == 0) return blocks;
+// CTAs so far; returns the new number.  size (log2 - 2): those of one size only.
+int res_add(ResTable& t, int blocks, const int32_t* items, const PicDesc* pic, const int32_t (&n)[4], int size = -1) {
+    if (size < 0 ? n[0] + n[1] + n[2] + n[3] == 0 : n[size] == 0) return blocks;
     ResSeg& sg = t.s[t.n++];
     sg.items = reinterpret_cast<const uint32_t*>(items);
+    for (int k = 3; size >= 0 && k > size; k--) sg.items += n[k];
     sg.pic = pic;
     sg.block0 = blocks;
     for (int k = 0; k < 4; k++) {
-        sg.n[k] = n[k];
-        blocks += res_blocks(n[k], k + 2);
+        sg.n[k] = size < 0 || k == size ? n[k] : 0;
+        blocks += res_blocks(sg.n[k], k + 2);
     }
     return blocks;
+}
+
+// Whether the blocks lie one after another in the pool, so that none shares samples with another.
+bool blocks_in_order(const hevc_tu_t* tus, int n) {
+    uint64_t end = 0;
+    bool ordered = true;
+    for (int i = 0; i < n; i++) {
+        ordered &= tus[i].coeff_offset >= end;
+        end = (uint64_t)tus[i].coeff_offset + ((uint64_t)1 << 2 * tus[i].log2_size);
+    }
+    return ordered;
 }
 
 // Parts (a power of two) that the strips of an MC launch are divided into, each a thread's.  A
@@ -1662,14 +1698,20 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
     }
     if (stages & (ST_RESID | ST_INTRA)) {
         StageMark m(ctx, ex.stream, 2);
-        for (int b0 = 0; b0 < n; b0 += MAX_SEGS) {
-            ResTable t;
-            std::memset(&t, 0, sizeof(t));
-            int blocks = 0;
-            for (int k = b0; k < std::min(n, b0 + MAX_SEGS); k++)
-                blocks = res_add(t, blocks, jobs[k]->d_res, jobs[k]->d_desc, jobs[k]->n_res);
-            if ((rc = L.go(k_residual, dim3(blocks), dim3(RES_THREADS), t, res_mode))) return rc;
-        }
+        // Blocks that cover samples of another (damaged streams; a caller's pool) are added size
+        // by size, 4x4 first: a launch of their own each, after the one for all other pictures.
+        bool by_size = false;
+        for (int k = 0; k < n; k++) by_size |= jobs[k]->res_by_size;
+        for (int size = -1; size < (by_size ? 4 : 0); size++)
+            for (int b0 = 0; b0 < n; b0 += MAX_SEGS) {
+                ResTable t;
+                std::memset(&t, 0, sizeof(t));
+                int blocks = 0;
+                for (int k = b0; k < std::min(n, b0 + MAX_SEGS); k++)
+                    if (jobs[k]->res_by_size == (size >= 0))
+                        blocks = res_add(t, blocks, jobs[k]->d_res, jobs[k]->d_desc, jobs[k]->n_res, size);
+                if ((rc = L.go(k_residual, dim3(blocks), dim3(RES_THREADS), t, res_mode))) return rc;
+            }
     }
     for (const IntraLaunch& g : intra) {
         StageMark m(ctx, ex.stream, 3);
@@ -1885,6 +1927,7 @@ int hevcgpu_residual_blocks_scaled(hevcgpu_ctx_t* ctx, const hevc_scaling_t* sca
     D.scaling = scaling ? reinterpret_cast<const hevc_scaling_t*>(base + o_scal) : nullptr;
     for (int k = 0; k < 4; k++) j.n_res[k] = (int32_t)bins[k].size();
     j.d_res = reinterpret_cast<const int32_t*>(base + o_res);
+    j.res_by_size = !blocks_in_order(tus, num_tus);
     CUDA_TRY(cudaMemcpyAsync(j.recs.p, j.pin.p, img, cudaMemcpyHostToDevice, ctx->stream));
     std::memcpy(static_cast<uint8_t*>(j.pin.p) + j.desc_off, &D, sizeof(D));
     CUDA_TRY(cudaMemcpyAsync(j.desc.p, static_cast<uint8_t*>(j.pin.p) + j.desc_off, sizeof(D),
@@ -2015,11 +2058,14 @@ int hevcgpu_residual_blocks_static(hevcgpu_ctx_t* ctx, const hevc_tu_t* tus, int
                              cudaMemcpyHostToDevice, ctx->stream));
 
     Launcher L{ctx, ctx->stream};
-    ResTable t;
-    std::memset(&t, 0, sizeof(t));
-    const int blocks = res_add(t, 0, reinterpret_cast<const int32_t*>(base + STATIC_LISTS_OFF),
-                               reinterpret_cast<const PicDesc*>(base), count);
-    if ((rc = L.go(k_residual, dim3(blocks), dim3(RES_THREADS), t, (int)RES_PACKED))) return rc;
+    const bool ordered = blocks_in_order(tus, num_tus);
+    for (int size = ordered ? -1 : 0; size < (ordered ? 0 : 4); size++) {   // as in run_stages
+        ResTable t;
+        std::memset(&t, 0, sizeof(t));
+        const int blocks = res_add(t, 0, reinterpret_cast<const int32_t*>(base + STATIC_LISTS_OFF),
+                                   reinterpret_cast<const PicDesc*>(base), count, size);
+        if ((rc = L.go(k_residual, dim3(blocks), dim3(RES_THREADS), t, (int)RES_PACKED))) return rc;
+    }
     // the lock is held until the kernels are done with the scratch (and `drained` waits
     // again on the way out of every earlier return)
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
