@@ -27,7 +27,7 @@ DROPIN_SO = os.path.join(PKG, "libhevcdec_gpu.so")
 DROPIN_CLI = os.path.join(PKG, "dropin", "_build", "hevc-decode")
 
 GPU_SOURCES = ["hevcgpu.cu"]
-GPU_DEPS = ["hevcgpu.cu", "kernels.cuh", "filters.cuh", "mc.cuh", "intra.cuh", "intra_levels.cuh", "intra_plan.h",
+GPU_DEPS = ["hevcgpu.cu", "kernels.cuh", "dequant.h", "filters.cuh", "mc.cuh", "intra.cuh", "intra_levels.cuh", "intra_plan.h",
             "device_common.cuh", "../../include/hevcgpu.h"]
 
 

@@ -8,6 +8,7 @@
 //   k_picture_checksum  per-plane checksum of a frame (H.265 picture hash SEI, D.3.19)
 #pragma once
 
+#include "dequant.h"
 #include "device_common.cuh"
 
 namespace hevcgpu {
@@ -103,30 +104,13 @@ __device__ __forceinline__ void idct_pairs(const uint32_t* x, int round, int* ds
     }
 }
 
-// Dequantisation of levels (transform.cpp:360-365): the product with m * levelScale[qP % 6], the
-// shift by qP / 6 and the rounding shift by s = 3 + log2 size, modulo 2^32, int16 clip.  With
-// qP / 6 < s the two shifts are one rounding shift by the difference (the product has as many
-// zeros at its end as the first put there, and |level * 255 * 72| stays below 2^30); else the
-// second undoes a part of the first.  Both forms: (level * (m * scale) + add) >> rs.
-struct Dequant {
-    int scale, add, rs;
-};
 __constant__ int c_level_scale[6] = {40, 45, 51, 57, 64, 72};
-__device__ __forceinline__ Dequant dequant_of(int qp, int log2) {
-    const int per = qp / 6, d = 3 + log2 - per;
-    Dequant q;
-    q.scale = c_level_scale[qp - 6 * per] << max(-d, 0);
-    q.rs = max(d, 0);
-    q.add = d > 0 ? 1 << (d - 1) : 0;
-    return q;
-}
+__device__ __forceinline__ Dequant dequant_of(int qp, int log2) { return dequant_make(c_level_scale[qp % 6], qp, log2); }
 // Levels of one column in two rows, each row's two columns in a word: the columns' pairs.
 __device__ __forceinline__ void dequant_pairs(uint32_t a, uint32_t b, const Dequant& q, int ma0, int ma1, int mb0, int mb1,
                                               uint32_t& p0, uint32_t& p1) {
-    const int a0 = ((int)(int16_t)a * (ma0 * q.scale) + q.add) >> q.rs, a1 = (((int)a >> 16) * (ma1 * q.scale) + q.add) >> q.rs;
-    const int b0 = ((int)(int16_t)b * (mb0 * q.scale) + q.add) >> q.rs, b1 = (((int)b >> 16) * (mb1 * q.scale) + q.add) >> q.rs;
-    p0 = pack_sat_s16x2(a0, b0);
-    p1 = pack_sat_s16x2(a1, b1);
+    p0 = pack_sat_s16x2(dequant_level((int16_t)a, ma0, q), dequant_level((int16_t)b, mb0, q));
+    p1 = pack_sat_s16x2(dequant_level((int)a >> 16, ma1, q), dequant_level((int)b >> 16, mb1, q));
 }
 
 // Scaling factors m (transform.cpp:320-358): matrixId is the plane plus 3 for a non-intra CU
