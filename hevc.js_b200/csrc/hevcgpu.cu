@@ -641,7 +641,8 @@ struct BuildScratch {
     std::vector<int2> itu_res;
     std::vector<IntraCtu> ictu;
     std::vector<uint32_t> watch_geo;
-    std::vector<uint16_t> items;
+    std::vector<uint16_t> items;   // the first n_items; like deps and dep_out it only grows
+    size_t n_items = 0, n_dep_out = 0;
     // A picture that k_intra_levels does, its TUs level by level (PicDesc::level_task), and per 4x4
     // unit the levels up to its last writer and its last reader.
     bool by_levels = false;
@@ -776,21 +777,23 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
     auto& itu_dep = BS.itu_dep;
     auto& dep_out = BS.dep_out;
     auto& ictu_watch = BS.ictu_watch;
+    // (arrays of which every entry is written below keep their old ones until then)
     ictu_addr.clear();
-    ictu_watch.clear();
     BS.ictu.clear();
     BS.watch.clear();
     BS.watch_geo.clear();
-    BS.items.clear();
     ictu_tu_off.clear();
-    itu.clear();
-    itu_rec.clear();
-    itu_res.clear();
-    itu_dep.clear();
-    dep_out.clear();
+    itu.resize((size_t)n_intra);
+    itu_rec.resize((size_t)n_intra);
+    itu_res.resize((size_t)n_intra);
+    itu_dep.resize((size_t)n_intra);
+    BS.n_items = BS.n_dep_out = 0;
     BS.depth = 0;
     BS.by_levels = false;
-    if (!n_intra) return HEVCGPU_OK;
+    if (!n_intra) {
+        ictu_watch.clear();
+        return HEVCGPU_OK;
+    }
     bool larger = false;   // than its CTB
     bool twice = false;    // covers a unit that another does
     BS.intra.clear(W, H);
@@ -825,74 +828,90 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
         const size_t nu = (size_t)uw[c] * uh[c];
         if (owner[c].size() < nu) owner[c].resize(nu, 0u);
     }
+    int last_ctu = 0;   // the last in raster order so far
     for (int b = 0; b < n_intra; b++) {
         const hevc_tu_t& t = s->tus[intra_list[(size_t)b]];
         const int c = t.c_idx, n = 1 << t.log2_size, sub = c ? 2 : 1;
         const int a = ((t.y * sub) >> p.log2_ctb) * wctb + ((t.x * sub) >> p.log2_ctb);
         ctu_of[(size_t)b] = a;
+        last_ctu = std::max(last_ctu, a);
         dep_at[(size_t)b] = (int32_t)n_own;
         if (n_own + 34 > deps.size()) {
             deps.resize(deps.size() * 2);
             D = deps.data();
         }
-        const size_t first_dep = n_own;
         uint32_t* own = owner[c].data();
         const int row = uw[c];
         int dp = 0;
-        uint32_t last = 0;   // a run of units with one owner adds what its first unit added
-        int32_t spare = 0, *last_at = &spare;
+        const size_t first = n_own;
+        size_t at_last = n_own;   // the entry of `last` (one more than there are: not kept)
+        uint32_t last = 0;
         // seg: the part of b's reference array the unit lies in (SEG_*); an owner's entry carries
-        // all parts it owns samples of
+        // all parts it owns samples of.  The units come along the array, so that those of one
+        // owner follow each other (blocks that do not overlap are squares) and only overlapping
+        // blocks need the search.
         auto dep = [&](uint32_t o, uint32_t seg) {
-            if ((o & GEN_BITS) != gtag) return;
             if (o == last) {
-                *last_at |= (int32_t)(seg << INTRA_DEP_SEG_SHIFT);
+                D[at_last] |= (int32_t)(seg << INTRA_DEP_SEG_SHIFT);
                 return;
             }
+            if ((o & GEN_BITS) != gtag) return;
             last = o;
-            last_at = &spare;
+            at_last = n_own;
             const int32_t ob = (int32_t)(o & 0xFFFFFFu);
-            const int oa = ctu_of[(size_t)ob];
             // a CTU later in raster order is never available to this one
             // (intra_prediction.cpp:113); in tile scan one can be decoded earlier (the
             // tile to the left, below-left), and waiting for it could wait for a CTA not
             // yet started: CTAs take CTUs in raster order
-            if (oa > a) return;
-            for (size_t q = first_dep; q < n_own; q++)
+            if (a < last_ctu && ctu_of[(size_t)ob] > a) return;
+            for (size_t q = first; twice && q < n_own; q++)
                 if ((D[q] & OWNER) == ob) {
                     D[q] |= (int32_t)(seg << INTRA_DEP_SEG_SHIFT);
-                    last_at = &D[q];
+                    at_last = q;
                     return;
                 }
-            last_at = &D[n_own];
             D[n_own++] = ob | (int32_t)(seg << INTRA_DEP_SEG_SHIFT);
             dp = std::max(dp, level[(size_t)ob] + 1);   // local and external dependencies alike
         };
         const int ux = t.x / 4, uy = t.y / 4, nu = n / 4;
-        if (uy > 0) {
-            const uint32_t* r = own + (size_t)(uy - 1) * row;
-            if (ux > 0) dep(r[ux - 1], SEG_C);
-            for (int x = ux; x < ux + nu; x++) dep(r[x], SEG_T);
-            for (int x = ux + nu; x < std::min(row, ux + 2 * nu); x++) dep(r[x], SEG_TR);
-        }
-        if (ux > 0) {
-            const uint32_t* r = own + (size_t)uy * row + ux - 1;
-            for (int y = 0; y < nu; y++, r += row) dep(*r, SEG_L);
-            for (int y = uy + nu; y < std::min(uh[c], uy + 2 * nu); y++, r += row) dep(*r, SEG_BL);
+        const uint32_t mark = gtag | (uint32_t)b;
+        uint32_t* const at = own + (size_t)uy * row + ux;
+        const bool left = ux > 0, above = uy > 0;
+        if (left && above) dep(at[-row - 1], SEG_C);
+        const uint32_t corner = n_own > first ? last : 0u;
+        if (nu == 1) {   // most TUs: no loops
+            if (above) {
+                dep(at[-row], SEG_T);
+                if (ux + 1 < row) dep(at[-row + 1], SEG_TR);
+            }
+            if (left) {
+                if (corner) last = corner, at_last = first;
+                dep(at[-1], SEG_L);
+                if (uy + 1 < uh[c]) dep(at[row - 1], SEG_BL);
+            }
+            at[0] = mark;
+        } else {
+            if (above) {
+                const uint32_t* r = at - row;
+                for (int x = 0; x < nu; x++) dep(r[x], SEG_T);
+                for (int x = nu; x < std::min(row - ux, 2 * nu); x++) dep(r[x], SEG_TR);
+            }
+            if (left) {
+                if (corner) last = corner, at_last = first;
+                const uint32_t* r = at - 1;
+                for (int y = 0; y < nu; y++, r += row) dep(*r, SEG_L);
+                for (int y = nu; y < std::min(uh[c] - uy, 2 * nu); y++, r += row) dep(*r, SEG_BL);
+            }
+            for (int y = 0; y < nu; y++)
+                for (int x = 0; x < nu; x++) at[(size_t)y * row + x] = mark;
         }
         level[(size_t)b] = dp;
         BS.depth = std::max(BS.depth, dp + 1);
-        const uint32_t mark = gtag | (uint32_t)b;
         larger |= n * sub > ctb;
         twice |= BS.intra.mark(t);
-        for (int y = uy; y < uy + n / 4; y++) {
-            uint32_t* r = own + (size_t)y * row;
-            for (int x = ux; x < ux + n / 4; x++) r[x] = mark;
-        }
     }
     BS.by_levels = larger || twice;
     dep_at[(size_t)n_intra] = (int32_t)n_own;
-    deps.resize(n_own);
     // Task order: CTUs in wavefront order (key 2 * row + column, then raster), each
     // CTU's TUs by depth (every TU after the TUs it depends on, and about in the order
     // they can run), then decode order.  CTAs take CTUs by ticket in this order, so
@@ -944,7 +963,6 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
     }
     auto& pos = BS.pos;   // decode order -> task order
     pos.resize((size_t)n_intra);
-    itu.resize((size_t)n_intra);
     for (int i = 0; i < n_intra; i++) {
         const int b = order[(size_t)i];
         pos[(size_t)b] = i;
@@ -962,11 +980,8 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
     // their first dependent TU comes, each get a watch slot, and the entry names the slot
     // (INTRA_DEP_WATCH).  Earlier CTUs come first, so the records those entries mark are
     // already written.
-    itu_res.assign((size_t)n_intra, make_int2(0, 0));
     int res_total = 0;
-    itu_rec.resize((size_t)n_intra);
-    itu_dep.resize((size_t)n_intra);
-    dep_out.resize(deps.size() + 1);   // one entry per owner found, and the spare entry
+    if (dep_out.size() <= n_own) dep_out.resize(n_own + 1);   // one entry per owner found, and the spare entry
     uint32_t* dout = dep_out.data();
     uint32_t nd = 0;
     const int nic = (int)ictu_addr.size();
@@ -989,7 +1004,7 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
     ictu_watch.assign((size_t)nic, 0u);
     slot_of.assign((size_t)n_intra, -1);
     int n_item = 0;
-    BS.items.resize((size_t)n_intra * intra_bands(5));
+    if (BS.items.size() < (size_t)n_intra * intra_bands(5)) BS.items.resize((size_t)n_intra * intra_bands(5));
     uint16_t* items = BS.items.data();
     for (int k = 0; k < nic; k++) {
         int acc = 0, nw = 0;
@@ -1035,6 +1050,7 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
             items[n_item++] = (uint16_t)(i - t0);
             for (int band = 1; band < intra_bands(t.log2_size); band++)
                 items[n_item++] = (uint16_t)((i - t0) | band << INTRA_DEP_TASK_SHIFT);
+            itu_res[(size_t)i] = make_int2(0, 0);
             if (!(t.flags & HEVC_TU_CODED)) continue;
             const int nn = 1 << (2 * t.log2_size);
             itu_res[(size_t)i] = make_int2((int)t.coeff_offset, res_total + acc);
@@ -1048,14 +1064,14 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
                            n_item - item0});
         res_total += acc;
     }
-    BS.items.resize((size_t)n_item);
+    BS.n_items = (size_t)n_item;
     BS.res_total = res_total;
     // one spare entry: an external dependency of task 0 on itself (the planted wait of
     // hevcgpu_job_plant_unmet_wait points task 0's list at it)
     *spare_dep = nd;
     dout[nd++] = INTRA_DEP_EXTERNAL | 0u;
-    dep_out.resize(nd);
-    if (dep_out.size() >= (1u << 26)) return fail(HEVCGPU_EINVAL, "intra dependency lists too long");
+    BS.n_dep_out = nd;
+    if (nd >= (1u << 26)) return fail(HEVCGPU_EINVAL, "intra dependency lists too long");
     return HEVCGPU_OK;
 }
 
@@ -1251,12 +1267,12 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     if (BS.by_levels) {   // no CTU of it goes to k_intra_ctus
         build_intra_levels(BS, s);
         ictu.clear();
-        BS.items.clear();
+        BS.n_items = 0;
         BS.watch_geo.clear();
     }
     j->n_level_items = (int32_t)BS.level_task.size();
     j->n_ictu = (int32_t)ictu.size();
-    j->n_items = (int32_t)BS.items.size();
+    j->n_items = (int32_t)BS.n_items;
     j->depth = BS.depth;
     for (int i = 0; i < n_intra; i++)
         if (itu_rec[(size_t)i].flags & HEVC_TU_CODED)
@@ -1288,8 +1304,8 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
         o_itu = pk.add(itu_rec.data(), sizeof(hevc_tu_t) * itu_rec.size());
         o_iro = pk.add(itu_res.data(), sizeof(int2) * itu_res.size());
         o_idp = pk.add(itu_dep.data(), sizeof(uint32_t) * itu_dep.size());
-        o_dl = pk.add(dep_out.data(), sizeof(uint32_t) * dep_out.size());
-        o_it = pk.add(BS.items.data(), sizeof(uint16_t) * BS.items.size());
+        o_dl = pk.add(dep_out.data(), sizeof(uint32_t) * BS.n_dep_out);
+        o_it = pk.add(BS.items.data(), sizeof(uint16_t) * BS.n_items);
         o_wl = pk.add(BS.watch_geo.data(), sizeof(uint32_t) * BS.watch_geo.size());
         o_lt = pk.add(BS.level_task.data(), sizeof(int2) * BS.level_task.size());
     };
@@ -1315,9 +1331,9 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
     size_t o_task = 0, o_wplan = 0, o_rev = 0, o_edge = 0;
     const size_t o_state = plan.add(nullptr, j->n_level_items ? IL_STATE * sizeof(int32_t) : 0);
     if (j->n_ictu) {
-        o_task = plan.add(nullptr, sizeof(IntraTask) * BS.items.size());
+        o_task = plan.add(nullptr, sizeof(IntraTask) * BS.n_items);
         o_wplan = plan.add(nullptr, sizeof(uint2) * BS.watch_geo.size());
-        o_rev = plan.add(nullptr, sizeof(uint16_t) * (dep_out.size() + 2));
+        o_rev = plan.add(nullptr, sizeof(uint16_t) * (BS.n_dep_out + 2));
         o_edge = plan.add(nullptr, (size_t)IC_EDGES * ictu.size());
     }
     rc = j->scratch.get(ctx, std::max<size_t>(plan.size, 256));
@@ -2374,7 +2390,8 @@ int hevcgpu_intra_schedule(const hevc_picture_syntax_t* syn, hevc_intra_schedule
     if ((rc = build_intra_schedule(BS, syn, &spare))) return rc;
     BS.task_flags.resize(BS.itu_rec.size());
     for (size_t i = 0; i < BS.itu_rec.size(); i++) BS.task_flags[i] = BS.itu_rec[i].reserved[0];
-    for (uint32_t& e : BS.dep_out) {   // the form the caller reads
+    for (size_t k = 0; k < BS.n_dep_out; k++) {   // the form the caller reads
+        uint32_t& e = BS.dep_out[k];
         const uint32_t q = e & INTRA_DEP_SOURCE;
         e = q < (uint32_t)IC_MAX_TUS ? q : INTRA_DEP_WATCH | (q - (uint32_t)IC_MAX_TUS);
     }
