@@ -1199,10 +1199,9 @@ int big_send_staged(hevcgpu_job* j, const BigArrays& b, Up&& up) {
     return HEVCGPU_OK;
 }
 
-// big_in: the large arrays, already laid out (big_begin) and the page-locked ones sent by
-// another thread; null: done here.
-int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool wait_uploads = true,
-              bool defer = false, const BigArrays* big_in = nullptr) {
+// big: the large arrays, laid out (big_begin) and the page-locked ones sent, or by another thread.
+int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, const BigArrays& big, bool wait_uploads,
+              bool defer) {
     BuildScratch& BS = t_build;
     hevcgpu_ctx* ctx = j->ctx;
     const hevc_pic_params_t& p = s->params;
@@ -1217,14 +1216,8 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, bool w
         j->ops.push_back(o);
         return HEVCGPU_OK;
     };
-    BigArrays local;
-    int rc;
-    if (!big_in) {
-        if ((rc = big_begin(j, s, local)) || (rc = big_send_direct(j, local))) return rc;
-        big_in = &local;
-    }
-    const BigArrays& big = *big_in;
-    if ((rc = big_send_staged(j, big, up))) return rc;
+    int rc = big_send_staged(j, big, up);
+    if (rc) return rc;
     const bool any_direct = big.any_direct;
 
     // residual bins (coded TUs by size) and the intra TUs in decode order
@@ -2105,8 +2098,9 @@ int run_host_picture(hevcgpu_ctx* ctx, const hevc_picture_syntax_t* syn, int sta
                      const uint8_t* const* refs, int num_refs, uint8_t* out) {
     hevcgpu_job j;
     j.ctx = ctx;
-    int rc = job_build(&j, syn, stages);
-    if (rc) return rc;
+    BigArrays big;
+    int rc = big_begin(&j, syn, big);
+    if (rc || (rc = big_send_direct(&j, big)) || (rc = job_build(&j, syn, stages, big, true, false))) return rc;
     const Layout& L = j.lay;
     std::vector<DevBuf> ref_bufs((size_t)std::max(0, num_refs));
     const uint8_t* ref_ptrs[2][16] = {};
@@ -2331,12 +2325,7 @@ int hevcgpu_slot_device_ptr(hevcgpu_stream_t* st, int32_t slot, void** y, void**
 }
 
 namespace {
-// defer: the job's CUDA calls stay queued in it for job_issue (batched preparation).
-// j, big: the job and its large arrays as batched preparation began them; null: begun here.
-int job_prepare(hevcgpu_stream_t* st, const hevc_picture_syntax_t* syn, hevcgpu_job_t** out, bool wait_uploads,
-                bool defer = false, hevcgpu_job* j = nullptr, const BigArrays* big = nullptr) {
-    if (!st || !out) return fail(HEVCGPU_EINVAL, "null arguments");
-    *out = nullptr;
+int job_check(hevcgpu_stream_t* st, const hevc_picture_syntax_t* syn) {
     int rc = check_ctx(st->ctx);
     if (rc) return rc;
     if ((rc = validate(syn, true, true, true))) return rc;
@@ -2349,29 +2338,38 @@ int job_prepare(hevcgpu_stream_t* st, const hevc_picture_syntax_t* syn, hevcgpu_
             if (s < 0 || s >= (int)st->slots.size())
                 return fail(HEVCGPU_EINVAL, "reference list %d entry %d names slot %d", l, i, s);
         }
-    const bool begun = j != nullptr;
-    if (!begun) {
-        j = new (std::nothrow) hevcgpu_job();
-        if (!j) return fail(HEVCGPU_ENOMEM, "host allocation");
-        j->ctx = st->ctx;
-        j->st = st;
-    }
-    if ((rc = job_build(j, syn, ST_ALL, wait_uploads, defer, big))) {
-        if (!begun) delete j;
-        return rc;
-    }
-    {
-        std::lock_guard<std::mutex> g(st->ctx->jobs_mu);
-        st->ctx->live_jobs.insert(j);
-        j->registered = true;
-    }
-    *out = j;
     return HEVCGPU_OK;
+}
+
+// The picture's job, its large arrays laid out.
+int job_begin(hevcgpu_stream_t* st, const hevc_picture_syntax_t* syn, std::unique_ptr<hevcgpu_job>& out, BigArrays& big) {
+    std::unique_ptr<hevcgpu_job> j(new (std::nothrow) hevcgpu_job());
+    if (!j) return fail(HEVCGPU_ENOMEM, "host allocation");
+    j->ctx = st->ctx;
+    j->st = st;
+    if (int rc = big_begin(j.get(), syn, big)) return rc;
+    out = std::move(j);
+    return HEVCGPU_OK;
+}
+
+// A job that is built belongs to the caller.
+hevcgpu_job_t* job_hand_out(std::unique_ptr<hevcgpu_job>& j) {
+    std::lock_guard<std::mutex> g(j->ctx->jobs_mu);
+    j->ctx->live_jobs.insert(j.get());
+    j->registered = true;
+    return j.release();
 }
 }  // namespace
 
 int hevcgpu_job_prepare(hevcgpu_stream_t* st, const hevc_picture_syntax_t* syn, hevcgpu_job_t** out) {
-    return job_prepare(st, syn, out, true);
+    if (!st || !out) return fail(HEVCGPU_EINVAL, "null arguments");
+    *out = nullptr;
+    std::unique_ptr<hevcgpu_job> j;
+    BigArrays big;
+    int rc = job_check(st, syn);
+    if (rc || (rc = job_begin(st, syn, j, big)) || (rc = big_send_direct(j.get(), big)) || (rc = job_build(j.get(), syn, ST_ALL, big, true, false))) return rc;
+    *out = job_hand_out(j);
+    return HEVCGPU_OK;
 }
 
 static_assert(HEVC_INTRA_DEP_WATCH == INTRA_DEP_WATCH && HEVC_INTRA_PUBLISH == ITU_PUBLISH,
@@ -2666,64 +2664,76 @@ int jobs_prepare(hevcgpu_stream_t* const* sts, const hevc_picture_syntax_t* cons
     std::vector<int> rcs((size_t)n, 0);
     std::vector<std::string> msgs((size_t)n);
     std::vector<BigArrays> big((size_t)n);
-    std::vector<std::unique_ptr<hevcgpu_job>> begun((size_t)n);   // with their large arrays laid out
-    for (int i = 0; i < n; i++) {
-        // (a picture that the checks will refuse is left to them)
-        const hevc_picture_syntax_t& p = *syns[i];
-        if (p.params.width != sts[i]->lay.W || p.params.height != sts[i]->lay.H || p.num_tus < 0 || p.num_pus < 0 ||
-            p.num_pus > MC_MAX_PUS)
-            continue;
-        std::unique_ptr<hevcgpu_job> j(new (std::nothrow) hevcgpu_job());
-        if (!j) continue;
-        j->ctx = ctx;
-        j->st = sts[i];
-        if ((rc = big_begin(j.get(), &p, big[(size_t)i]))) return fail(rc, "picture %d: %s", i, std::string(g_err).c_str());
-        begun[(size_t)i] = std::move(j);
-    }
+    std::vector<std::unique_ptr<hevcgpu_job>> jobs((size_t)n);
     {
         std::lock_guard<std::mutex> g(ctx->pool.run_mu);
         ctx->pool.ensure(ctx->device);
-        // One task sends the pictures' page-locked arrays and then, as the others build the
-        // jobs' host images, their other CUDA calls, picture by picture; it builds too while
-        // the next picture is not ready.  (8 1080p P/B pictures from host records to host
-        // frames: 4.35 ms with all calls made after the last image was built, 2.97 ms.)
+        // The workers take a picture each: check it, lay out its large arrays, build the job's host
+        // image.  One task meanwhile lays out and sends the arrays of the pictures that have
+        // some in page-locked memory, then makes their other CUDA calls as they are built; it builds
+        // too while the next picture is not ready.  (8 1080p P/B pictures from host records to host
+        // frames: 4.35 ms with all calls made after the last image was built, 2.85 ms.)  Pageable
+        // arrays, whose buffers take longer to get, are left to the workers.  What was found wrong
+        // with a picture's records counts before what its buffers or its uploads gave.
+        enum : int { NONE, TAKEN, BEGUN };
+        struct Progress {
+            std::atomic<int> begun{NONE};
+            std::atomic<bool> built{false};
+            int begin_rc = HEVCGPU_OK, send_rc = HEVCGPU_OK;
+            std::string begin_msg, send_msg;
+        };
+        std::vector<Progress> progress((size_t)n);
         std::atomic<int> next{0};
-        std::unique_ptr<std::atomic<bool>[]> built(new std::atomic<bool>[(size_t)n]);
-        for (int i = 0; i < n; i++) built[(size_t)i].store(false, std::memory_order_relaxed);
+        auto begin = [&](size_t k) {   // or waits until the other thread has
+            Progress& p = progress[k];
+            int none = NONE;
+            if (p.begun.compare_exchange_strong(none, TAKEN)) {
+                if ((p.begin_rc = job_begin(sts[k], syns[k], jobs[k], big[k]))) p.begin_msg = g_err;
+                p.begun.store(BEGUN, std::memory_order_release);
+            }
+            while (p.begun.load(std::memory_order_acquire) < BEGUN) std::this_thread::yield();
+        };
         auto build_one = [&]() {
-            const int i = next.fetch_add(1);
-            if (i >= n) return false;
-            const size_t k = (size_t)i;
-            rcs[k] = job_prepare(sts[k], syns[k], &out[k], wait_uploads, true, begun[k].get(), begun[k] ? &big[k] : nullptr);
-            if (rcs[k]) msgs[k] = g_err;
-            built[k].store(true, std::memory_order_release);
+            const size_t k = (size_t)next.fetch_add(1);
+            if (k >= (size_t)n) return false;
+            Progress& p = progress[k];
+            if ((rcs[k] = job_check(sts[k], syns[k]))) {
+                msgs[k] = g_err;
+            } else {
+                begin(k);
+                if ((rcs[k] = p.begin_rc)) msgs[k] = p.begin_msg;
+                else if ((rcs[k] = job_build(jobs[k].get(), syns[k], ST_ALL, big[k], wait_uploads, true))) msgs[k] = g_err;
+            }
+            p.built.store(true, std::memory_order_release);
             return true;
         };
-        int sent = HEVCGPU_OK, issued = HEVCGPU_OK;
-        std::string sent_msg;
         ctx->pool.run(n + 1, [&](int t) {
             if (t > 0) {
                 build_one();
                 return;
             }
-            for (int k = 0; k < n && !sent; k++)
-                if (begun[(size_t)k] && (sent = big_send_direct(begun[(size_t)k].get(), big[(size_t)k]))) sent_msg = g_err;
-            for (int k = 0; k < n; k++) {
-                while (!built[(size_t)k].load(std::memory_order_acquire))
+            for (size_t k = 0; k < (size_t)n; k++) {
+                const hevc_picture_syntax_t& s = *syns[k];
+                if (s.params.width != sts[k]->lay.W || s.params.height != sts[k]->lay.H || s.num_tus < 0 || s.num_pus < 0 ||
+                    s.num_pus > MC_MAX_PUS ||   // (will be refused)
+                    !(page_locked(s.pus) || page_locked(s.blk) || page_locked(s.tus) || page_locked(s.coeffs)))
+                    continue;
+                begin(k);
+                Progress& p = progress[k];
+                if (jobs[k] && (p.send_rc = big_send_direct(jobs[k].get(), big[k]))) p.send_msg = g_err;
+            }
+            bool ok = true;
+            for (size_t k = 0; k < (size_t)n; k++) {
+                Progress& p = progress[k];
+                while (!p.built.load(std::memory_order_acquire))
                     if (!build_one()) std::this_thread::yield();
-                if (rcs[(size_t)k] || issued || sent) continue;
-                if ((issued = rcs[(size_t)k] = job_issue(out[k]))) msgs[(size_t)k] = g_err;
+                if (!rcs[k] && (rcs[k] = p.send_rc)) msgs[k] = p.send_msg;
+                if (ok && !rcs[k] && (rcs[k] = job_issue(jobs[k].get()))) msgs[k] = g_err;
+                ok = ok && !rcs[k];
             }
         });
         for (int i = 0; i < n; i++)
-            if (out[i]) begun[(size_t)i].release();   // the caller's from here on
-        if (sent)
-            for (int i = 0; i < n; i++)
-                if (!rcs[(size_t)i]) {
-                    rcs[(size_t)i] = sent;
-                    msgs[(size_t)i] = sent_msg;
-                    break;
-                }
+            if (!rcs[(size_t)i]) out[i] = job_hand_out(jobs[(size_t)i]);
     }
     for (int i = 0; i < n; i++) {
         if (!rcs[(size_t)i]) continue;
