@@ -260,6 +260,7 @@ struct hevcgpu_ctx {
     cudaEvent_t done[EVENT_RING] = {};
     int done_next = 0;
     cudaEvent_t next_done() { cudaEvent_t e = done[done_next]; done_next = (done_next + 1) % EVENT_RING; return e; }
+    std::atomic<int> lanes{0};   // open lanes
     std::mutex jobs_mu;
     std::set<hevcgpu_job*> live_jobs;   // jobs of the DPB API, for lanes that close
     // Reads and clears the sticky device status of a flow area; maps it to a return code.
@@ -1530,7 +1531,11 @@ struct Launcher {
 // Dynamic shared memory of a loop filter launch: as much as leaves room for just the per_sm CTAs
 // an SM has to take.  The launch may start while the intra stage still holds most SMs, and would
 // otherwise put all of a small launch's CTAs on the few that are free: 4 streams' GOPs at 720p
-// (960 tiles a launch) 1,160 us without it, 1,125 with it.
+// (960 tiles a launch) 1,160 us without it, 1,125 with it.  Only where the context has one
+// queue: the CTAs that wait would keep the CTAs of another queue's kernels off their SMs.  GOPs
+// of 8 over two and four lanes, frames/s with it and without: 4 streams of 416x240 a lane
+// 94,500 / 127,500 and 135,000 / 177,500; one of 1280x720 14,400 / 17,100 and 18,200 / 20,600, four
+// 37,000 / 40,000 and 42,000 / 46,300; two of 1080p 15,800 / 17,100 and 17,300 / 19,500.
 size_t lf_pad(int per_sm, int threads) {
     if (per_sm >= lf_ctas(threads)) return 0;
     return (228 * 1024 / per_sm - 1024 - sizeof(LfSmem)) & ~(size_t)127;
@@ -1602,6 +1607,7 @@ struct StageMark {
 struct Exec {
     cudaStream_t stream;
     void* flow;
+    bool alone;   // no other queue of the context is open (the context's stream counts as one only for its own launches)
     int32_t* tickets() const { return reinterpret_cast<int32_t*>(static_cast<uint8_t*>(flow) + sizeof(FlowState) + 16); }
 };
 
@@ -1762,7 +1768,7 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
             [&](dim3 grid, const SegTable& t, int tiles) {
                 const int per_sm = (tiles + ctx->sm_count - 1) / ctx->sm_count, deblock = stages & ST_DEBLOCK ? 1 : 0;
                 auto go = [&](auto* kernel, int threads) {
-                    return L.go_smem(kernel, grid, dim3(threads), lf_pad(per_sm, threads), t, deblock);
+                    return L.go_smem(kernel, grid, dim3(threads), ex.alone ? lf_pad(per_sm, threads) : 0, t, deblock);
                 };
                 // 256 threads while all tiles are resident at once, else 128 (lf_ctas)
                 if (per_sm <= lf_ctas(256)) return go(k_loop_filter<256>, 256);
@@ -1774,7 +1780,7 @@ int run_stages(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, int n
 }
 
 int run_stages(hevcgpu_ctx* ctx, hevcgpu_job* const* jobs, int n, int stages, int res_mode) {
-    return run_stages(ctx, Exec{ctx->stream, ctx->flow}, jobs, n, stages, res_mode);
+    return run_stages(ctx, Exec{ctx->stream, ctx->flow, ctx->lanes == 0}, jobs, n, stages, res_mode);
 }
 
 // Copies between a pitched slot and a packed I420 host frame.  When the pitches equal the
@@ -2572,14 +2578,14 @@ int launch_batch(hevcgpu_ctx* ctx, const Exec& ex, cudaEvent_t done, hevcgpu_job
 int hevcgpu_job_launch(hevcgpu_job_t* job, int32_t dst_slot) {
     if (!job) return fail(HEVCGPU_EINVAL, "null job");
     hevcgpu_job* jp = job;
-    return launch_batch(job->ctx, Exec{job->ctx->stream, job->ctx->flow}, job->ctx->next_done(), &jp, &dst_slot, 1);
+    return launch_batch(job->ctx, Exec{job->ctx->stream, job->ctx->flow, job->ctx->lanes == 0}, job->ctx->next_done(), &jp, &dst_slot, 1);
 }
 
 int hevcgpu_batch_launch(hevcgpu_job_t* const* jobs, const int32_t* dst_slots, int32_t n) {
     hevcgpu_ctx* ctx = nullptr;
     int rc = check_batch(jobs, dst_slots, n, &ctx);
     if (rc) return rc;
-    return launch_batch(ctx, Exec{ctx->stream, ctx->flow}, ctx->next_done(), jobs, dst_slots, n);
+    return launch_batch(ctx, Exec{ctx->stream, ctx->flow, ctx->lanes == 0}, ctx->next_done(), jobs, dst_slots, n);
 }
 
 // ---- lanes ---------------------------------------------------------------------------
@@ -2605,6 +2611,7 @@ int hevcgpu_lane_open(hevcgpu_ctx_t* ctx, hevcgpu_lane_t** out) {
         delete ln;
         return fail(HEVCGPU_ECUDA, "lane set-up: %s", cudaGetErrorString(e));
     }
+    ctx->lanes++;
     *out = ln;
     return HEVCGPU_OK;
 }
@@ -2622,6 +2629,7 @@ void hevcgpu_lane_close(hevcgpu_lane_t* lane) {
                 j->last_done = nullptr;
             }
     }
+    lane->ctx->lanes--;
     delete lane;
 }
 
@@ -2635,7 +2643,7 @@ int hevcgpu_lane_batch_launch(hevcgpu_lane_t* lane, hevcgpu_job_t* const* jobs, 
     // the jobs' record uploads and the slots' uploads ran on the context's stream
     CUDA_TRY(cudaEventRecord(lane->ctx_ready, ctx->stream));
     CUDA_TRY(cudaStreamWaitEvent(lane->stream, lane->ctx_ready, 0));
-    return launch_batch(ctx, Exec{lane->stream, lane->flow}, lane->next_done(), jobs, dst_slots, n);
+    return launch_batch(ctx, Exec{lane->stream, lane->flow, ctx->lanes == 1}, lane->next_done(), jobs, dst_slots, n);
 }
 
 int hevcgpu_lane_sync(hevcgpu_lane_t* lane) {
