@@ -555,12 +555,11 @@ def run_ours(args, hb, rank, world, local):
                         "frac_of_hbm": round(gbs / peak, 4)}
     dom = max(stage_ms, key=lambda k: stage_ms[k])
     # DRAM bytes (read + write) per batch of each stage's kernels on this workload, from one
-    # ncu capture of a GOP of 2 streams at 1080p (ncu --metrics dram__bytes_read.sum,
+    # ncu capture of a GOP of its 8 streams (ncu --metrics dram__bytes_read.sum,
     # dram__bytes_write.sum --clock-control none python bench.py --profile-only --steps 1
-    # --warmup 0 --streams 2), scaled by 4 to 8 pictures per launch (each picture is
-    # independent work), the GOP's total divided by its 60 batches; taken again whenever the
-    # stage's kernels change
-    ncu_dram_gop8 = {"mc": 59200734, "residual": 47180459, "intra": 30119697, "loop_filter": 37424230}
+    # --warmup 0): which form of a kernel runs depends on the pictures in a batch.  The GOP's
+    # total divided by its 60 batches; taken again whenever the stage's kernels change
+    ncu_dram_gop8 = {"mc": 58776175, "residual": 47083874, "intra": 30140612, "loop_filter": 37921254}
     traffic = (ncu_dram_gop8[dom] if dom in ncu_dram_gop8 and (W, H, G, F) == (W_DEFAULT, H_DEFAULT, 8, 60)
                else None)
 

@@ -135,8 +135,8 @@ struct PicDesc {
 // when the kernel before has completed; every kernel calls it, at the latest before it ends,
 // so a kernel that has passed it knows that all kernels before it are done.  The first kernel
 // of a batch is launched without the attribute: it starts when everything before it is done,
-// and pdl_wait returns at once.  One 416x240 P/B picture 93 -> 58 us, one 1080p 128 -> 92,
-// 16 in a batch 503 -> 468.
+// and pdl_wait returns at once.  One 416x240 P/B picture 93 -> 57 us, one 1080p 128 -> 95,
+// 16 in a batch 503 -> 485.
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -166,15 +166,16 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // A launch covers up to MAX_SEGS pictures.  Segment k owns the blocks
 // [block0, next block0) of an item-list launch, or blockIdx.y == k of a per-picture
 // launch (whose items field is the picture the loop filter writes).  The table is a kernel
-// parameter, so a batched launch needs no device-side bookkeeping and is captured by value in a
-// CUDA graph.
+// parameter, so a batched launch needs no device-side bookkeeping.  (A graph that held one would
+// replay the epoch of its intra launch, and take the border words of the launch before for new.)
 constexpr int MAX_SEGS = 64;
 struct Seg {
     const void* items;
     const PicDesc* pic;
     int32_t n_items;
     int32_t block0;
-    int32_t aux0, aux1;   // per-launch extras (aux1 of an intra launch: its epoch)
+    int32_t epoch;   // of an intra launch
+    int32_t pad;
 };
 struct SegTable {
     int32_t n;

@@ -393,10 +393,10 @@ struct hevcgpu_stream {
 // jobs: one picture's records, prepared and uploaded
 // ---------------------------------------------------------------------------------------
 // A CUDA call of a job's preparation: a host->device copy, zeroing device memory, or
-// recording the event that marks the copies straight from the caller's arrays as done.
-// Prepared on the context's host workers, the calls are queued in the job and issued by
-// the thread that asked for the batch, so that the workers make no CUDA calls (which would
-// contend for the driver's locks) and every upload goes out from one thread in order.
+// recording the event that marks the copies straight from the caller's arrays as done.  In
+// batched preparation the workers that build the jobs queue these calls in them, and one task of
+// the batch, on whichever thread took it, issues them all (calls from every worker contend for
+// the driver's locks).  Workers make CUDA calls only to get buffers.
 struct UploadOp {
     enum Kind : int { COPY, ZERO, MARK_DIRECT } kind;
     void* dst;
@@ -443,9 +443,8 @@ struct hevcgpu_job {
     hevc_pic_params_t params{};
     ~hevcgpu_job() {
         // buffers go back to the pools only after every queued use of them has run: a job's
-        // uploads all precede its launches (the launching stream waits for the context
-        // stream, and descriptor copies go on the launching stream), so the completion of its
-        // last batch covers them; a job never launched waits for the context stream
+        // uploads are all on the context's stream, which a launching lane waits for first, so the
+        // completion of its last batch covers them; a job never launched waits for that stream
         if (last_done) cudaEventSynchronize(last_done);   // the job's last batch, not later ones
         else if (last_stream) cudaStreamSynchronize(last_stream);
         else if (ctx) cudaStreamSynchronize(ctx->stream);
@@ -1635,8 +1634,7 @@ int intra_warps(int ctus, int64_t items, int depth, int deep_ctus, int64_t deep_
 }
 
 // The intra launches of a batch, one per group of up to MAX_SEGS pictures: CTAs take intra CTUs
-// by ticket in wavefront order per picture; block0 = intra CTUs of earlier pictures, aux1 =
-// epoch.
+// by ticket in wavefront order per picture; block0 = intra CTUs of earlier pictures.
 struct IntraLaunch {
     SegTable t;
     int total;
@@ -1661,7 +1659,7 @@ int intra_launches(hevcgpu_ctx* ctx, const Exec& ex, hevcgpu_job* const* jobs, i
                 CUDA_TRY(cudaMemsetAsync(j->host_desc.edge, 0, j->edge_bytes, ex.stream));
                 j->epoch = 0;
             }
-            sg.aux1 = ++j->epoch;
+            sg.epoch = ++j->epoch;
             total += j->n_ictu;
             items += j->n_items;
             if (j->depth > depth) {
@@ -2379,7 +2377,7 @@ int hevcgpu_job_prepare(hevcgpu_stream_t* st, const hevc_picture_syntax_t* syn, 
 }
 
 static_assert(HEVC_INTRA_DEP_WATCH == INTRA_DEP_WATCH && HEVC_INTRA_PUBLISH == ITU_PUBLISH,
-              "the schedule the diagnostic hands out is the one the kernel reads");
+              "the diagnostic's flags are the kernel's");
 
 int hevcgpu_intra_schedule(const hevc_picture_syntax_t* syn, hevc_intra_schedule_t* out) {
     if (!out) return fail(HEVCGPU_EINVAL, "null out");

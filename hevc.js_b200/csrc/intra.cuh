@@ -256,7 +256,7 @@ constexpr int IC_EDGE_L = 1 + 3 * 16, IC_EDGE_C = 1 + 3 * 8;
 constexpr int IC_EDGES = 128;                        // >= IC_EDGE_L + 2 * IC_EDGE_C, 4 per watcher lane
 constexpr int IC_TILES = IC_LH * IC_LP + 2 * IC_CH * IC_CP;   // bytes of the three tiles; then a byte 128
 constexpr unsigned long long WAIT_LIMIT_NS = 1000000000ull;   // a wait gives up after a second
-constexpr unsigned SPIN_LIMIT = 1u << 26;            // backstop: polls of at least 64 ns
+constexpr unsigned SPIN_LIMIT = 1u << 26;            // polls, should the timer not advance
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(32 * WARPS, ic_ctas(WARPS)) k_intra_ctus(const
     }
     const int k = S.pic_index;
     const PicDesc& P = *st.s[k].pic;
-    const int32_t epoch = st.s[k].aux1;
+    const int32_t epoch = st.s[k].epoch;
     // the CTU's record: the same 16-byte loads by every thread, and no chain of loads after it
     const int4* const cp = reinterpret_cast<const int4*>(static_cast<const IntraCtu*>(st.s[k].items) + S.ticket);
     const int4 c0 = __ldg(cp), c1 = __ldg(cp + 1), c2 = __ldg(cp + 2);
