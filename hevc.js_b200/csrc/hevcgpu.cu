@@ -2670,47 +2670,37 @@ int jobs_prepare(hevcgpu_stream_t* const* sts, const hevc_picture_syntax_t* cons
     std::vector<int> rcs((size_t)n, 0);
     std::vector<std::string> msgs((size_t)n);
     std::vector<BigArrays> big((size_t)n);
-    std::vector<std::unique_ptr<hevcgpu_job>> jobs((size_t)n);
+    std::vector<std::unique_ptr<hevcgpu_job>> jobs((size_t)n);   // with their large arrays laid out
+    // What is found wrong with a picture's records counts before what its buffers or its uploads
+    // gave, so failures of those are kept until the picture has been checked.
+    std::vector<int> begun((size_t)n, HEVCGPU_OK), sent((size_t)n, HEVCGPU_OK);
+    std::vector<std::string> begun_msgs((size_t)n), sent_msgs((size_t)n);
+    for (size_t k = 0; k < (size_t)n; k++) {
+        // (a picture that the checks will refuse is left to them)
+        const hevc_picture_syntax_t& p = *syns[k];
+        if (p.params.width != sts[k]->lay.W || p.params.height != sts[k]->lay.H || p.num_tus < 0 || p.num_pus < 0 ||
+            p.num_pus > MC_MAX_PUS)
+            continue;
+        if ((begun[k] = job_begin(sts[k], syns[k], jobs[k], big[k]))) begun_msgs[k] = g_err;
+    }
     {
         std::lock_guard<std::mutex> g(ctx->pool.run_mu);
         ctx->pool.ensure(ctx->device);
-        // The workers take a picture each: check it, lay out its large arrays, build the job's host
-        // image.  One task meanwhile lays out and sends the arrays of the pictures that have
-        // some in page-locked memory, then makes their other CUDA calls as they are built; it builds
-        // too while the next picture is not ready.  (8 1080p P/B pictures from host records to host
-        // frames: 4.35 ms with all calls made after the last image was built, 2.85 ms.)  Pageable
-        // arrays, whose buffers take longer to get, are left to the workers.  What was found wrong
-        // with a picture's records counts before what its buffers or its uploads gave.
-        enum : int { NONE, TAKEN, BEGUN };
-        struct Progress {
-            std::atomic<int> begun{NONE};
-            std::atomic<bool> built{false};
-            int begin_rc = HEVCGPU_OK, send_rc = HEVCGPU_OK;
-            std::string begin_msg, send_msg;
-        };
-        std::vector<Progress> progress((size_t)n);
+        // One task sends the pictures' page-locked arrays and then, as the others build the
+        // jobs' host images, their other CUDA calls, picture by picture; it builds too while
+        // the next picture is not ready.  (8 1080p P/B pictures from host records to host
+        // frames: 4.35 ms with all calls made after the last image was built, 2.85 ms; the same
+        // with the large arrays laid out by the workers.)
         std::atomic<int> next{0};
-        auto begin = [&](size_t k) {   // or waits until the other thread has
-            Progress& p = progress[k];
-            int none = NONE;
-            if (p.begun.compare_exchange_strong(none, TAKEN)) {
-                if ((p.begin_rc = job_begin(sts[k], syns[k], jobs[k], big[k]))) p.begin_msg = g_err;
-                p.begun.store(BEGUN, std::memory_order_release);
-            }
-            while (p.begun.load(std::memory_order_acquire) < BEGUN) std::this_thread::yield();
-        };
+        std::vector<std::atomic<bool>> built((size_t)n);
+        for (auto& x : built) x.store(false, std::memory_order_relaxed);
         auto build_one = [&]() {
             const size_t k = (size_t)next.fetch_add(1);
             if (k >= (size_t)n) return false;
-            Progress& p = progress[k];
-            if ((rcs[k] = job_check(sts[k], syns[k]))) {
-                msgs[k] = g_err;
-            } else {
-                begin(k);
-                if ((rcs[k] = p.begin_rc)) msgs[k] = p.begin_msg;
-                else if ((rcs[k] = job_build(jobs[k].get(), syns[k], ST_ALL, big[k], wait_uploads, true))) msgs[k] = g_err;
-            }
-            p.built.store(true, std::memory_order_release);
+            if ((rcs[k] = job_check(sts[k], syns[k]))) msgs[k] = g_err;
+            else if ((rcs[k] = begun[k])) msgs[k] = begun_msgs[k];
+            else if ((rcs[k] = job_build(jobs[k].get(), syns[k], ST_ALL, big[k], wait_uploads, true))) msgs[k] = g_err;
+            built[k].store(true, std::memory_order_release);
             return true;
         };
         ctx->pool.run(n + 1, [&](int t) {
@@ -2718,22 +2708,13 @@ int jobs_prepare(hevcgpu_stream_t* const* sts, const hevc_picture_syntax_t* cons
                 build_one();
                 return;
             }
-            for (size_t k = 0; k < (size_t)n; k++) {
-                const hevc_picture_syntax_t& s = *syns[k];
-                if (s.params.width != sts[k]->lay.W || s.params.height != sts[k]->lay.H || s.num_tus < 0 || s.num_pus < 0 ||
-                    s.num_pus > MC_MAX_PUS ||   // (will be refused)
-                    !(page_locked(s.pus) || page_locked(s.blk) || page_locked(s.tus) || page_locked(s.coeffs)))
-                    continue;
-                begin(k);
-                Progress& p = progress[k];
-                if (jobs[k] && (p.send_rc = big_send_direct(jobs[k].get(), big[k]))) p.send_msg = g_err;
-            }
+            for (size_t k = 0; k < (size_t)n; k++)
+                if (jobs[k] && (sent[k] = big_send_direct(jobs[k].get(), big[k]))) sent_msgs[k] = g_err;
             bool ok = true;
             for (size_t k = 0; k < (size_t)n; k++) {
-                Progress& p = progress[k];
-                while (!p.built.load(std::memory_order_acquire))
+                while (!built[k].load(std::memory_order_acquire))
                     if (!build_one()) std::this_thread::yield();
-                if (!rcs[k] && (rcs[k] = p.send_rc)) msgs[k] = p.send_msg;
+                if (!rcs[k] && (rcs[k] = sent[k])) msgs[k] = sent_msgs[k];
                 if (ok && !rcs[k] && (rcs[k] = job_issue(jobs[k].get()))) msgs[k] = g_err;
                 ok = ok && !rcs[k];
             }
