@@ -470,10 +470,10 @@ struct Packer {
         return off;
     }
     // lists by size, largest first, back to back
-    size_t add_joined(const std::vector<int32_t> (&lists)[4]) {
+    size_t add_joined(const std::vector<int32_t> (&lists)[4], const int32_t (&n)[4]) {
         const size_t off = add(nullptr, 0);
         for (int k = 3; k >= 0; k--) {
-            const size_t bytes = sizeof(int32_t) * lists[k].size();
+            const size_t bytes = sizeof(int32_t) * (size_t)n[k];
             if (out && bytes) std::memcpy(out + size, lists[k].data(), bytes);
             size += bytes;
         }
@@ -601,8 +601,7 @@ enum StageMask : int {
 };
 
 // The 4x4 units that blocks of a picture cover, a bit each.  A block lies at a multiple of its size,
-// so the 64 units of 32x32 samples are a word and a block is one mask (a loop over a block's rows
-// cost a 1080p P/B picture 4 % of its preparation).
+// so the 64 units of 32x32 samples are a word and a block is one mask.
 struct UnitMap {
     std::vector<uint64_t> words[3];
     int pitch[3] = {0, 0, 0};
@@ -612,12 +611,12 @@ struct UnitMap {
             words[c].assign((size_t)pitch[c] * (size_t)(((c ? H / 2 : H) + 31) / 32), 0);
         }
     }
-    // Marks a block's units; true if some were marked already.
-    bool mark(const hevc_tu_t& t) {
+    // Marks a block's units if `on` is 1 (nothing if 0); those that were marked already.
+    uint64_t mark(const hevc_tu_t& t, uint32_t on) {
         static constexpr uint64_t block[4] = {1ull, 0x303ull, 0x0F0F0F0Full, ~0ull};
-        const uint64_t m = block[t.log2_size - 2] << ((t.y & 28) * 2 + (t.x & 28) / 4);
+        const uint64_t m = (block[t.log2_size - 2] << ((t.y & 28) * 2 + (t.x & 28) / 4)) & (0 - (uint64_t)on);
         uint64_t& w = words[t.c_idx][(size_t)(t.y >> 5) * pitch[t.c_idx] + (t.x >> 5)];
-        const bool hit = (w & m) != 0;
+        const uint64_t hit = w & m;
         w |= m;
         return hit;
     }
@@ -628,7 +627,9 @@ struct UnitMap {
 // the context), so that their memory is reused from one picture to the next: no allocation
 // and no first-touch page faults per picture.
 struct BuildScratch {
-    std::vector<int32_t> bins[4], intra_list, itu, level, ctu_of, order;
+    std::vector<int32_t> bins[4];   // coded TUs by size: as many of each as are counted in n_bin
+    int32_t n_bin[4] = {0, 0, 0, 0};
+    std::vector<int32_t> intra_list, itu, level, ctu_of, order;
     UnitMap coded, intra;   // units that coded inter TUs and intra TUs cover
     // intra owner maps, one word per 4x4 unit: (generation << 24) | decode-order index of the
     // intra TU.  An entry is valid when its generation is this picture's, so the maps need
@@ -908,7 +909,7 @@ int build_intra_schedule(BuildScratch& BS, const hevc_picture_syntax_t* s, uint3
         level[(size_t)b] = dp;
         BS.depth = std::max(BS.depth, dp + 1);
         larger |= n * sub > ctb;
-        twice |= BS.intra.mark(t);
+        twice |= BS.intra.mark(t, 1u) != 0;
     }
     BS.by_levels = larger || twice;
     dep_at[(size_t)n_intra] = (int32_t)n_own;
@@ -1220,25 +1221,34 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, const 
     if (rc) return rc;
     const bool any_direct = big.any_direct;
 
-    // residual bins (coded TUs by size) and the intra TUs in decode order
+    // Residual bins (coded TUs by size) and the intra TUs in decode order.  No branches: which kind a
+    // TU is cannot be predicted.  Each list has room for all TUs, and one more that is not kept.
     auto& bins = BS.bins;
     auto& intra_list = BS.intra_list;
-    for (auto& v : bins) v.clear();
-    intra_list.clear();
-    for (auto& v : bins) v.reserve((size_t)s->num_tus / 2);
-    intra_list.reserve((size_t)s->num_tus);
-    bool twice = false;   // two coded inter TUs cover a unit
-    if (stages & ST_RESID) BS.coded.clear(W, H);
-    for (int i = 0; i < s->num_tus; i++) {
-        const hevc_tu_t& t = s->tus[i];
-        bool intra = t.flags & HEVC_TU_INTRA;
-        if ((t.flags & HEVC_TU_CODED) && !intra && (stages & ST_RESID)) {
-            bins[t.log2_size - 2].push_back(i);
-            twice |= BS.coded.mark(t);
-        }
-        if (intra && (stages & ST_INTRA)) intra_list.push_back(i);
+    auto& n_bin = BS.n_bin;
+    const int n_tus = stages & (ST_RESID | ST_INTRA) ? s->num_tus : 0;   // (else they have not been checked)
+    const size_t room = (size_t)n_tus + 1;
+    for (int k = 0; k < 4; k++) {
+        if (bins[k].size() < room) bins[k].resize(room);
+        n_bin[k] = 0;
     }
-    j->res_by_size = twice;
+    if (intra_list.size() < room) intra_list.resize(room);
+    const uint32_t all_inter = stages & ST_RESID ? 1u : 0u, all_intra = stages & ST_INTRA ? 1u : 0u;
+    uint64_t twice = 0;   // units that two coded inter TUs cover
+    int n_intra = 0;
+    BS.coded.clear(W, H);
+    for (int i = 0; i < n_tus; i++) {
+        const hevc_tu_t& t = s->tus[i];
+        const uint32_t intra = t.flags & HEVC_TU_INTRA, coded = (uint32_t)(t.flags >> 1) & ~intra & all_inter;
+        int32_t& n = n_bin[t.log2_size - 2];
+        bins[t.log2_size - 2][(size_t)n] = i;
+        n += (int)coded;
+        intra_list[(size_t)n_intra] = i;
+        n_intra += (int)(intra & all_intra);
+        twice |= BS.coded.mark(t, coded);
+    }
+    intra_list.resize((size_t)n_intra);
+    j->res_by_size = twice != 0;
     j->has_intra = !intra_list.empty();
     // Intra schedule.  Per plane an owner map at 4-sample granularity records the latest
     // intra TU written there; intra TU B reads the units of its reference row
@@ -1249,7 +1259,6 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, const 
     // not use (availability) can only add an unneeded wait, never change a sample; owners in
     // CTUs later in raster order (decoded earlier only in tile scan) are never available
     // and add nothing.
-    const int n_intra = (int)intra_list.size();
     auto& ictu = BS.ictu;               // the CTUs' records
     auto& itu_rec = BS.itu_rec;         // intra TU records in task order
     auto& itu_res = BS.itu_res;         // per task entry of a coded TU: offsets of its levels and residual
@@ -1269,7 +1278,8 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, const 
     j->depth = BS.depth;
     for (int i = 0; i < n_intra; i++)
         if (itu_rec[(size_t)i].flags & HEVC_TU_CODED)
-            bins[itu_rec[(size_t)i].log2_size - 2].push_back((int32_t)(RES_INTRA_ITEM | (uint32_t)i));
+            bins[itu_rec[(size_t)i].log2_size - 2][(size_t)n_bin[itu_rec[(size_t)i].log2_size - 2]++] =
+                (int32_t)(RES_INTRA_ITEM | (uint32_t)i);
     // MC strips (build_mc_strips)
     auto& mc = BS.mc;
     if (stages & ST_MC) build_mc_strips(BS, s, j->lay.pitch_y, j->lay.pitch_c);
@@ -1291,7 +1301,7 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, const 
         o_ti = pk.add(s->ctb_tile, s->ctb_tile ? sizeof(uint16_t) * (size_t)nctb : 0);
         o_slices = s->num_slices > 0 && s->slices ? pk.add(s->slices, sizeof(hevc_slice_t) * (size_t)s->num_slices)
                                                   : pk.add(&dflt, sizeof(dflt));
-        o_res = pk.add_joined(bins);
+        o_res = pk.add_joined(bins, BS.n_bin);
         for (int c = 0; c < 2; c++) o_mc[c] = pk.add(mc[c].data(), sizeof(uint32_t) * mc[c].size());
         o_ia = pk.add(ictu.data(), sizeof(IntraCtu) * ictu.size());
         o_itu = pk.add(itu_rec.data(), sizeof(hevc_tu_t) * itu_rec.size());
@@ -1399,7 +1409,7 @@ int job_build(hevcgpu_job* j, const hevc_picture_syntax_t* s, int stages, const 
         }
     }
     D.pcm_bypass_any = pcm_bypass ? 1 : 0;
-    for (int k = 0; k < 4; k++) j->n_res[k] = (int32_t)bins[k].size();
+    for (int k = 0; k < 4; k++) j->n_res[k] = n_bin[k];
     j->d_res = reinterpret_cast<const int32_t*>(base + o_res);
     for (int c = 0; c < 2; c++) {
         j->n_mc[c] = (int32_t)mc[c].size();
@@ -1917,6 +1927,7 @@ int hevcgpu_residual_blocks_scaled(hevcgpu_ctx_t* ctx, const hevc_scaling_t* sca
     j.ctx = ctx;
     std::vector<int32_t> bins[4];
     for (int i = 0; i < num_tus; i++) bins[tus[i].log2_size - 2].push_back(i);
+    for (int k = 0; k < 4; k++) j.n_res[k] = (int32_t)bins[k].size();
     size_t o_tus, o_coef, o_pred, o_out, o_res, o_scal = 0;
     auto pack = [&](Packer& pk) {
         if (scaling) o_scal = pk.add(scaling, sizeof(hevc_scaling_t));
@@ -1924,7 +1935,7 @@ int hevcgpu_residual_blocks_scaled(hevcgpu_ctx_t* ctx, const hevc_scaling_t* sca
         o_coef = pk.add(coeffs, sizeof(int16_t) * (size_t)num_coeffs);
         o_pred = pk.add(pred, (size_t)num_coeffs);
         o_out = pk.add(nullptr, (size_t)num_coeffs);
-        o_res = pk.add_joined(bins);
+        o_res = pk.add_joined(bins, j.n_res);
     };
     Packer measure;
     pack(measure);
@@ -1944,7 +1955,6 @@ int hevcgpu_residual_blocks_scaled(hevcgpu_ctx_t* ctx, const hevc_scaling_t* sca
     D.rec = base + o_pred;
     D.dst = base + o_out;
     D.scaling = scaling ? reinterpret_cast<const hevc_scaling_t*>(base + o_scal) : nullptr;
-    for (int k = 0; k < 4; k++) j.n_res[k] = (int32_t)bins[k].size();
     j.d_res = reinterpret_cast<const int32_t*>(base + o_res);
     j.res_by_size = !blocks_in_order(tus, num_tus);
     CUDA_TRY(cudaMemcpyAsync(j.recs.p, j.pin.p, img, cudaMemcpyHostToDevice, ctx->stream));
