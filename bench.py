@@ -44,7 +44,8 @@ dropin     the drop-in decoder (hevc_decoder_decode, CABAC included) on the refe
            same on generated 1080p random-access streams, without and with WPP, in a child
            process bounded by a timeout.
 --impl reference runs privaloops/hevc.js's own reconstruction functions (oracle/_ref,
-           compiled from the reference's sources) on all host cores for the same GOP mix.
+           compiled from the reference's sources) on all host cores for the same GOP mix, and
+           reports it as unavailable where they are not built.
 """
 import argparse
 import json
@@ -368,9 +369,11 @@ def run_reference(args, hb, rank, world):
     reconstructs the next `batch` pictures of the GOP work list."""
     if rank != 0:
         return None
+    checker, kind = cpu_checker()
+    if kind != "reference":   # the restatement in oracle/ is not the reference
+        return {"impl": "reference", "unavailable": "oracle/_ref/libhevcref.so is not built: it takes the reference's sources"}
     W, H, G, F, B = args.width, args.height, args.streams, args.gop, args.batch
     seq = gop_sequence(make_gop(hb, G, W, H, rank_seed0(0)), F)
-    checker, kind = cpu_checker()
     threads = os.cpu_count() or 1
     pos = 0
     for _ in range(args.warmup):
