@@ -397,7 +397,10 @@ __global__ void __launch_bounds__(IP_THREADS) k_intra_plan(const __grid_constant
 #pragma unroll 1
     for (int q = tid; q < n_tu + n_watch; q += IP_THREADS) s_count[source(q)] = 0;
     if (tid < IC_EDGES / 4) reinterpret_cast<uint32_t*>(s_edge)[tid] = 0xFFFFFFFFu;
-    if (tid == 0) s_total = s_bad = 0;
+    if (tid == 0) {
+        s_total = 0;
+        s_bad = C.n_tu > IC_MAX_TUS || C.n_watch > IC_MAX_WATCH || C.n_dep > IC_DEP_STAGE || C.n_item > IC_MAX_TUS;
+    }
 #pragma unroll 1
     for (int i = tid; i < n_tu; i += IP_THREADS) {
         const hevc_tu_t t = P.itu_rec[C.tu_first + i];
