@@ -16,8 +16,7 @@ MAX_ITEMS, MAX_ENTRIES = 384, 2048   # work items and dependency entries of a CT
 
 
 class Records:
-    """A generated picture with other TUs: dicts of hevc_tu_t fields, coded ones with the levels
-    of TU `like` of the generated picture."""
+    """A generated picture with other TUs, given as dicts of hevc_tu_t fields."""
 
     def __init__(self, hb, pic, tus):
         self.base = pic
