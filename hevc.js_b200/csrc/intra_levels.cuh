@@ -6,23 +6,23 @@
 // IC_MAX_TUS work items and IC_DEP_STAGE dependencies, and a border word has one writer.  Here
 // the host sorts a picture's TUs into levels by what decode order asks for (build_intra_levels):
 // a TU comes after the writers of every sample it reads or covers and after the readers of every
-// sample it covers.  Warps take the TUs (those of 16x16 and 32x32 in
-// bands of 8 rows) level by level, and start one when all of the levels before have completed,
-// which one counter per picture tells.  So nothing is sized by
-// how often a block is coded.  Reference samples come from the picture, each with its own
-// availability, since a TU may reach past its CTB.
+// sample it covers.  Warps take the TUs (those of 16x16 and 32x32 in bands of 8 rows) level by
+// level, and start one when all of the levels before have completed, which one counter per
+// picture tells.  So nothing is sized by how often a block is coded.  Reference samples come from
+// the picture, each with its own availability, since a TU may reach past its CTB.
 //
 // Bound by the levels, one after another: a counter's round trip through L2, reference samples
 // from L2, one item's work and its release, 5 us a level (a 1080p I picture with a few blocks coded
-// twice: 2,158 levels, 11 ms; 6.8 us a level with TUs not in bands).  64 to 256 warps a picture
-// make no difference.  Every wait is bounded as in intra.cuh.
+// twice: 2,158 levels, 11 ms; 14.8 ms with TUs not in bands).  64 to 256 warps a picture make no
+// difference to it; a P/B picture (87 levels) takes 0.86 ms with 64, 0.68 with 128, 0.61 with 256.
+// Every wait is bounded as in intra.cuh.
 #pragma once
 
 #include "intra.cuh"
 
 namespace hevcgpu {
 
-constexpr int IL_WARPS = 4, IL_CTAS = 32;   // per picture
+constexpr int IL_WARPS = 8, IL_CTAS = 32;   // per picture
 
 __global__ void __launch_bounds__(32 * IL_WARPS) k_intra_levels(const __grid_constant__ SegTable st, uint32_t* sticky) {
     constexpr uint32_t FULL = 0xffffffffu;
